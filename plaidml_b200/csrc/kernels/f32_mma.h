@@ -1,0 +1,53 @@
+// fp32 matrix products and convolutions on the bf16 tensor pipe, operands split on the way into shared memory.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <string>
+
+#include "tc_launch.h"
+
+namespace pmlb {
+
+// C[b][i][j] = sum_k A(b, i, k) * B(b, k, j), everything fp32 in device memory.
+struct F32MmaLaunch {
+  int m = 0, n = 0, k = 0, batch = 1;
+  const float* a = nullptr;
+  long long lda = 0, a_batch = 0;   // a_mn false: A(i, k) at a[i * lda + k]; true: at a[k * lda + i]
+  bool a_mn = false;
+  const ConvGeom* conv = nullptr;   // non-null: A is an NHWC activation at `a` (c a multiple of 4),
+                                    // row i = output pixel i, k = (tap, channel); m, n, k, batch = n*p*q, k_out, r*s*c, 1
+  const float* b = nullptr;
+  long long ldb = 0, b_batch = 0;   // b_mn false: B(k, j) at b[j * ldb + k]; true: at b[k * ldb + j]
+  bool b_mn = false;
+  float* out = nullptr;             // may be null with row maxima
+  long long ldc = 0, out_batch = 0;
+  int epi_flags = 0;                // kEpi*; bias f32[n], residual f32 rows ldr apart
+  const float* bias = nullptr;
+  const float* residual = nullptr;
+  long long ldr = 0, res_batch = 0;
+  float* rowmax = nullptr;          // f32[batch * m], filled with -inf by the caller
+  int* status = nullptr;            // device word that receives a non-zero code if a wait times out
+  int bn_override = 0;              // 0 = choose; else 64, 128 or 256
+  int split_override = 0;           // 0 = choose; else the number of CTAs (1..8) that share a tile's K range
+};
+
+// Whether the kernel accepts a convolution.
+bool f32_mma_takes_conv(const ConvGeom& g);
+
+// Whether the kernel is expected to be faster than splitting the operands into TF32 parts by pre-passes.
+struct F32MmaShape {
+  int m = 0, n = 0, k = 0, batch = 1;
+  bool conv = false;
+  bool aligned_in = true, aligned_out = true;   // rows start on 16-byte boundaries
+  long long elems = 0;                          // elements that each call's pre-pass would split
+};
+bool f32_mma_faster(const F32MmaShape& shape);
+
+// Returns 0 on success, otherwise a pmlb_status value with a message in *err.
+int f32_mma_launch(const F32MmaLaunch& launch, cudaStream_t stream, std::string* err);
+
+// Filter of an fp32 convolution as the kernel reads it: [taps][c][k] of f32, bf16 or f16 -> the same in f32.
+cudaError_t launch_filter_to_f32(const void* in, int in_dtype, float* out, long long elems, cudaStream_t stream);
+
+}  // namespace pmlb

@@ -8,6 +8,7 @@
 #include <new>
 #include <string>
 
+#include "f32_mma.h"
 #include "generic.h"
 #include "pmlb_kernels.h"
 #include "prepass.h"
@@ -95,10 +96,12 @@ struct pmlb_plan {
   bool owns_status = true;
 
   pmlb_gemm_desc gemm;
-  long long kpad = 0;       // fp32 path: padded K of the split copies
+  long long kpad = 0;       // transposed B, split fp32 operands: padded K or channel count
   bool transpose_b = false; // 8/16-bit path: B goes through [n][k] scratch
-  bool split = false;
+  bool f32_mma = false;     // fp32 operands split inside the kernel (f32_mma.cu)
+  bool split = false;       // fp32 operands split into TF32 parts by pre-passes
   int armed_wait_us = 0;    // > 0: the next invoke runs the time-out test (see pmlb_plan_arm_timeout_test)
+  bool ksplit_off = false;  // the caller (or the environment) wants K in one part
   int ksplit = 1;           // parts of the K range (two-pass split-K), each of kslice elements
   long long kslice = 0;
 
@@ -118,6 +121,16 @@ struct pmlb_plan {
 };
 
 namespace {
+
+pmlb::ConvGeom conv_geom(const pmlb_conv_desc& d) {
+  pmlb::ConvGeom g;
+  g.n = d.n; g.h = d.h; g.w = d.w; g.c = d.c;
+  g.r = d.r; g.s = d.s; g.p = d.p; g.q = d.q;
+  g.stride_h = d.stride_h; g.stride_w = d.stride_w;
+  g.pad_h = d.pad_h; g.pad_w = d.pad_w;
+  g.dil_h = d.dil_h; g.dil_w = d.dil_w;
+  return g;
+}
 
 pmlb_status alloc_plan_memory(pmlb_plan* plan, size_t scratch_bytes, bool need_status) {
   cudaGetDevice(&plan->device);
@@ -318,12 +331,22 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
   plan->kind_name = "tc_gemm";
   plan->gemm = *d;
   size_t scratch = 0;
+  const long long a_mats = d->stride_a != 0 ? d->batch : 1, b_mats = d->stride_b != 0 ? d->batch : 1;
   if (f32) {
-    plan->split = true;
-    plan->kpad = round_up(d->k, 4);
-    const long long a_mats = d->stride_a != 0 ? d->batch : 1;
-    const long long b_mats = d->stride_b != 0 ? d->batch : 1;
-    scratch = static_cast<size_t>(2 * 4 * plan->kpad * (a_mats * d->m + b_mats * d->n));
+    pmlb::F32MmaShape shape;
+    shape.m = d->m, shape.n = d->n, shape.k = d->k, shape.batch = d->batch;
+    shape.aligned_in = d->lda % 4 == 0 && d->ldb % 4 == 0;
+    shape.aligned_out = d->ldc % 4 == 0;
+    shape.elems = (a_mats * d->m + b_mats * d->n) * d->k;
+    // (a forced 256-wide tile is refused for f32, by the other route)
+    if ((d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_faster(shape)) {
+      plan->f32_mma = true;   // no scratch but the status word
+      scratch = 256;
+    } else {
+      plan->split = true;
+      plan->kpad = round_up(d->k, 4);
+      scratch = static_cast<size_t>(2 * 4 * plan->kpad * (a_mats * d->m + b_mats * d->n));
+    }
   } else {
     if ((d->lda * eb) % 16 != 0 || (d->stride_a * eb) % 16 != 0) {
       delete plan;
@@ -338,13 +361,13 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
     } else if ((d->flags & PMLB_GEMM_TRANSPOSE_B) || !b_aligned) {
       plan->transpose_b = true;
       plan->kpad = round_up(d->k, 16 / eb);
-      const long long b_mats = d->stride_b != 0 ? d->batch : 1;
       scratch = static_cast<size_t>(b_mats * d->n * plan->kpad * eb);
     }
   }
   // Split K?  (8/16-bit inputs read in place, one matrix, no row maxima: see PMLB_GEMM_NO_SPLIT_K)
   const char* split_env = std::getenv("PMLB_SPLIT_K");   // "0": never split (sums then never depend on the tile count)
   const bool split_allowed = !(split_env && split_env[0] == '0') || (d->flags & PMLB_GEMM_SPLIT_K);
+  plan->ksplit_off = !split_allowed || (d->flags & PMLB_GEMM_NO_SPLIT_K) != 0;
   if (!f32 && !plan->transpose_b && d->batch == 1 && !(d->epilogue & PMLB_EPI_ROWMAX) && d->k_first == 0 &&
       !(d->flags & PMLB_GEMM_NO_SPLIT_K) && split_allowed) {
     const int bk = 128 / eb;
@@ -368,14 +391,18 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
       }
     }
   }
-  pmlb_status st = alloc_plan_memory(plan, scratch, true);
+  pmlb_status st = alloc_plan_memory(plan, scratch, !plan->f32_mma);
   if (st != PMLB_OK) {
     pmlb_plan_free(plan);
     return st;
   }
-  if (plan->transpose_b && plan->scratch) {
-    // the K tail of the transposed copy must read as zero
+  if ((plan->transpose_b && plan->scratch) || plan->f32_mma) {
+    // the K tail of the transposed copy (the status word) must read as zero
     cudaMemset(plan->scratch, 0, plan->scratch_bytes);
+  }
+  if (plan->f32_mma) {
+    plan->status = static_cast<int*>(plan->scratch);
+    plan->owns_status = false;
   }
   *out = plan;
   return PMLB_OK;
@@ -401,6 +428,30 @@ pmlb_status pmlb_gemm_invoke_two(pmlb_plan* plan, void* stream_v, const void* a,
   if ((d.epilogue & PMLB_EPI_ROWMAX) && !rowmax) return fail(PMLB_ERR_INVALID, "gemm: rowmax missing");
   if (!(d.epilogue & PMLB_EPI_ROWMAX) && !c) return fail(PMLB_ERR_INVALID, "gemm: null output");
 
+  if (plan->f32_mma) {
+    pmlb::F32MmaLaunch f;
+    f.m = d.m, f.n = d.n, f.k = d.k, f.batch = d.batch;
+    f.a = static_cast<const float*>(a), f.lda = d.lda, f.a_batch = d.stride_a;
+    f.b = static_cast<const float*>(b), f.ldb = d.ldb, f.b_batch = d.stride_b;
+    f.b_mn = !d.b_is_nk;
+    f.out = static_cast<float*>(c), f.ldc = d.ldc, f.out_batch = d.stride_c;
+    f.epi_flags = d.epilogue;
+    f.bias = static_cast<const float*>(bias);
+    f.residual = (d.epilogue & PMLB_EPI_RESIDUAL) ? static_cast<const float*>(residual) : nullptr;
+    f.ldr = d.ldr, f.res_batch = d.stride_r;
+    f.rowmax = rowmax;
+    f.status = plan->status;
+    f.bn_override = d.tile_n;
+    if (plan->ksplit_off) f.split_override = 1;
+    if (d.epilogue & PMLB_EPI_ROWMAX) {
+      cudaError_t e = pmlb::launch_fill_f32(rowmax, static_cast<long long>(d.batch) * d.m, -__builtin_inff(), stream);
+      if (e != cudaSuccess) return cuda_fail(e, "fill(rowmax)");
+    }
+    std::string err;
+    const int rc = pmlb::f32_mma_launch(f, stream, &err);
+    if (rc != 0) return fail(static_cast<pmlb_status>(rc), "gemm: " + err);
+    return PMLB_OK;
+  }
   pmlb::TcLaunch L;
   L.elem_bytes = elem_bytes_of(d.in_dtype);
   L.is_f16 = d.in_dtype == PMLB_F16;
@@ -579,7 +630,16 @@ pmlb_status pmlb_conv_dispatch(const pmlb_conv_desc* d, pmlb_plan** out) {
   plan->kind_name = "tc_conv";
   plan->conv = *d;
   size_t scratch = static_cast<size_t>(d->k) * d->r * d->s * d->c * 2;
-  if (f32) {
+  pmlb::F32MmaShape shape;
+  shape.m = d->n * d->p * d->q, shape.n = d->k, shape.k = d->r * d->s * d->c;
+  shape.conv = true;
+  shape.aligned_in = shape.aligned_out = d->k % 4 == 0;
+  shape.elems = static_cast<long long>(d->n) * d->h * d->w * d->c;
+  if (f32 && (d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_takes_conv(conv_geom(*d)) &&
+      pmlb::f32_mma_faster(shape)) {
+    plan->f32_mma = true;
+    scratch = static_cast<size_t>(d->k) * d->r * d->s * d->c * 4;   // the filter, [r][s][c][k] in f32
+  } else if (f32) {
     // fp32: three TF32 products per term (as the fp32 GEMM): the filter and, per call, the activation are split
     // into high and low TF32 parts, channels padded to whole 16-byte groups; scratch = [w hi][w lo][x hi][x lo]
     plan->split = true;
@@ -631,7 +691,10 @@ pmlb_status pmlb_conv_set_filter(pmlb_plan* plan, void* stream, const void* filt
   }
   const pmlb_conv_desc& d = plan->conv;
   cudaError_t e;
-  if (plan->split) {
+  if (plan->f32_mma) {
+    e = pmlb::launch_filter_to_f32(filter, dtype, static_cast<float*>(plan->scratch),
+                                   static_cast<long long>(d.r) * d.s * d.c * d.k, static_cast<cudaStream_t>(stream));
+  } else if (plan->split) {
     const size_t wts = static_cast<size_t>(d.k) * d.r * d.s * plan->kpad;   // elements of one part
     e = pmlb::launch_filter_relayout_split(filter, dtype, static_cast<float*>(plan->scratch),
                                            static_cast<float*>(plan->scratch) + wts, d.r * d.s, d.c,
@@ -760,12 +823,25 @@ pmlb_status pmlb_conv_invoke(pmlb_plan* plan, void* stream, const void* input, v
     if (rc != 0) return fail(static_cast<pmlb_status>(rc), "conv (packed rows): " + err);
     return PMLB_OK;
   }
-  pmlb::ConvGeom g;
-  g.n = d.n; g.h = d.h; g.w = d.w; g.c = d.c;
-  g.r = d.r; g.s = d.s; g.p = d.p; g.q = d.q;
-  g.stride_h = d.stride_h; g.stride_w = d.stride_w;
-  g.pad_h = d.pad_h; g.pad_w = d.pad_w;
-  g.dil_h = d.dil_h; g.dil_w = d.dil_w;
+  pmlb::ConvGeom g = conv_geom(d);
+  if (plan->f32_mma) {
+    pmlb::F32MmaLaunch f;
+    f.m = d.n * d.p * d.q, f.n = d.k, f.k = d.r * d.s * d.c;
+    f.conv = &g;
+    f.a = static_cast<const float*>(input);
+    f.b = static_cast<const float*>(plan->scratch), f.ldb = d.k, f.b_mn = true;
+    f.out = static_cast<float*>(output), f.ldc = d.k;
+    f.epi_flags = d.epilogue;
+    f.bias = static_cast<const float*>(bias);
+    f.residual = (d.epilogue & PMLB_EPI_RESIDUAL) ? static_cast<const float*>(residual) : nullptr;
+    f.ldr = d.k;
+    f.status = plan->status;
+    f.bn_override = d.tile_n;
+    std::string err;
+    const int rc = pmlb::f32_mma_launch(f, static_cast<cudaStream_t>(stream), &err);
+    if (rc != 0) return fail(static_cast<pmlb_status>(rc), "conv: " + err);
+    return PMLB_OK;
+  }
   pmlb::TcLaunch L;
   L.elem_bytes = 2;
   L.is_f16 = d.in_dtype == PMLB_F16;

@@ -72,17 +72,31 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
                : "memory");
 }
 
+// CLUSTER: acquires at cluster scope, for barriers that threads of another CTA arrive on after writing shared memory.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  }
   return ok != 0;
 }
 
@@ -116,17 +130,18 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;
 // flag itself).  `abort_flag` lives in shared memory: word 0 is the flag, word 1 the code of
 // the role that gave up first (written by the callers), word 2 the wait limit of this launch in
 // microseconds (0 = kWaitLimitNs).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
 #pragma unroll 1
   for (int i = 0; i < 128; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
   }
   const uint64_t t0 = global_timer_ns();
 #pragma unroll 1
   while (true) {
 #pragma unroll 1
     for (int i = 0; i < 64; ++i) {
-      if (mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
     }
     if (*abort_flag != 0) return false;
     const uint64_t limit_us = static_cast<uint64_t>(abort_flag[2]);
@@ -139,9 +154,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // The same wait made by all 32 lanes of a warp, with one answer for the warp: false if any
 // lane gave up.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
                                                volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+  return __all_sync(0xffffffffu, mbar_wait<CLUSTER>(bar, parity, abort_flag)) != 0;
 }
 
 // ---------------------------------------------------------------- CTA pairs (clusters of two)

@@ -424,6 +424,56 @@ def test_f32_ragged():
     assert max_rel(c.cpu().numpy(), oracle.gemm_f32_acc64(a, b, False)) < 1e-5
 
 
+@pytest.mark.parametrize("m,n,k,b_is_nk,tile_n,offset", [
+    (1, 64, 64, False, 64, 0),          # one k-block, one row
+    (128, 128, 257, True, 128, 0),      # a second accumulator chain of one ragged block, rows not 16-byte aligned
+    (129, 65, 192, False, 64, 0),       # 3 k-blocks over 3 CTAs: strips of 43 rows
+    (200, 260, 448, False, 128, 1),     # 7 k-blocks over 7 CTAs, operands 4 bytes off alignment
+    (64, 100, 1030, True, 0, 0),        # K split with a ragged end
+    (2047, 2049, 513, False, 0, 0),     # CTA pairs, ragged in every dimension
+    (2047, 2052, 516, True, 0, 0),
+])
+def test_f32_operands_split_in_the_kernel(m, n, k, b_is_nk, tile_n, offset):
+    g = rng(3100 + m + k)
+    a = g.uniform(-1, 1, size=(1, m, k)).astype(np.float32)
+    b = g.uniform(-1, 1, size=(1, n, k) if b_is_nk else (1, k, n)).astype(np.float32)
+    bias = g.standard_normal(n).astype(np.float32)
+
+    def off(x):   # the same values `offset` elements into a buffer
+        buf = torch.zeros(x.size + offset, dtype=torch.float32, device="cuda")
+        buf[offset:] = torch.from_numpy(x.reshape(-1)).cuda()
+        return buf[offset:].view(x.shape)
+
+    c, _, plan = run_gemm(K.F32, K.F32, off(a), off(b), m, n, k, 1, b_is_nk, epilogue=K.EPI_BIAS | K.EPI_RELU, bias=dev(bias),
+                          tile_n=tile_n)
+    assert plan.scratch_bytes == 256    # the status word: no split copies
+    ref = np.maximum(oracle.gemm_f32_acc64(a, b, b_is_nk) + bias, 0)
+    # products keep 24 bits (2^-24 each); a chain of 16 (pairs: k / 16) truncating additions of at most 2^-23 of the
+    # largest partial sum, which a random walk leaves below twice the largest result
+    chain = 16 if m < 2000 else (k + 15) // 16
+    assert max_rel(c.cpu().numpy(), ref) < (2 * chain + 8) * 2.0 ** -23
+
+
+def test_f32_split_operands_keep_infinities_and_nan():
+    g = rng(3200)
+    m, n, k = 130, 70, 300
+    a = g.uniform(0.5, 1, size=(1, m, k)).astype(np.float32)
+    b = g.uniform(0.5, 1, size=(1, k, n)).astype(np.float32)
+    a[0, 3, 7] = np.inf
+    a[0, 5, 299] = -np.inf
+    a[0, 9, 0] = np.nan
+    a[0, 11, 1] = 3.0e38      # finite, its products with 1.5 of them overflow
+    b[0, 1, 2] = 1.5
+    c, _, _ = run_gemm(K.F32, K.F32, dev(a), dev(b), m, n, k, 1, False)
+    got = c.cpu().numpy()[0]
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = (a[0].astype(np.float64) @ b[0].astype(np.float64)).astype(np.float32)
+    assert np.all(got[3] == np.inf) and np.all(got[5] == -np.inf) and np.all(np.isnan(got[9]))
+    assert got[11, 2] == np.inf
+    rows = [r for r in range(m) if r not in (3, 5, 9, 11)]
+    assert max_rel(got[rows], want[rows]) < 1e-6
+
+
 # --- CTA pairs (two CTAs per 256 x 256 tile) -----------------------------------------------------
 
 @pytest.mark.parametrize("b_is_nk", [True, False], ids=["B[n][k]", "B[k][n]"])
