@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "pmlb_kernels.h"
+#include "tc_gemm.cuh"   // FastDiv
 
 namespace pmlb {
 
@@ -46,6 +47,31 @@ struct GenericParams {
   long long out_elems;
 };
 
+// The strided form of a contraction (contract_route.h fills it): offsets as sums of steps per output dim and per loop.
+struct LeanParams {
+  int rank, n_src, n_check;
+  int agg, combo, has_init, out_dtype, init_dtype;
+  int size[PMLB_MAX_RANK];
+  FastDiv fd_size[PMLB_MAX_RANK];
+  long long out_stride[PMLB_MAX_RANK];
+  long long init_stride[PMLB_MAX_RANK];
+  int loop[4];                  // extents of the loops, the innermost last
+  struct Source {
+    int base, dtype;
+    int out[PMLB_MAX_RANK];     // step per output dim
+    int loop[4];                // step per loop
+  } src[2];
+  struct Check {                // 0 <= base + steps < size
+    int base, size;
+    int out[PMLB_MAX_RANK];
+    int loop[4];
+  } check[4];
+  long long elems;
+  const void* srcp[2];
+  const void* initp;
+  void* outp;
+};
+
 enum : int {
   kEwIdent = 0, kEwAdd, kEwSub, kEwMul, kEwDiv, kEwMod, kEwMax, kEwMin, kEwNeg, kEwAbs, kEwRelu,
   kEwSign, kEwSelect, kEwCmpEq, kEwCmpNe, kEwCmpLt, kEwCmpLe, kEwCmpGt, kEwCmpGe, kEwLogicalAnd,
@@ -73,6 +99,7 @@ struct EltwiseParams {
 };
 
 cudaError_t launch_contract(const GenericParams& p, cudaStream_t stream);
+cudaError_t launch_contract_lean(const LeanParams& p, cudaStream_t stream);
 cudaError_t launch_eltwise(const EltwiseParams& p, cudaStream_t stream);
 cudaError_t launch_fill_f32(float* out, long long n, float value, cudaStream_t stream);
 

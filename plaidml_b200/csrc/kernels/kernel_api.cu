@@ -8,6 +8,7 @@
 #include <new>
 #include <string>
 
+#include "contract_route.h"
 #include "f32_mma.h"
 #include "generic.h"
 #include "pmlb_kernels.h"
@@ -116,6 +117,8 @@ struct pmlb_plan {
   pmlb_reduce_desc reduce;
   pmlb_pool_desc pool;
   pmlb::GenericParams generic;
+  bool lean = false;             // contraction: strided form (else the general kernel)
+  pmlb::LeanParams lean_params;
   pmlb::EltwiseParams eltwise;
   pmlb_special_desc special;
 };
@@ -1076,6 +1079,7 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
       if (!direct || !used[i]) p.loop_var[p.n_loop++] = i;
     }
   }
+  plan->lean = pmlb::lean_form(p, &plan->lean_params);
   cudaGetDevice(&plan->device);
   *out = plan;
   return PMLB_OK;
@@ -1084,15 +1088,26 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
 pmlb_status pmlb_contract_invoke(pmlb_plan* plan, void* stream, const void* src0, const void* src1,
                                  const void* src2, const void* init, void* outp) {
   if (!plan || plan->kind != kPlanContract) return fail(PMLB_ERR_INVALID, "not a contraction plan");
-  pmlb::GenericParams p = plan->generic;
+  const pmlb::GenericParams& g = plan->generic;
+  if (!outp || !src0 || (g.n_src > 1 && !src1) || (g.n_src > 2 && !src2) || (g.has_init && !init)) {
+    return fail(PMLB_ERR_INVALID, "contract: null tensor");
+  }
+  if (plan->lean) {
+    pmlb::LeanParams l = plan->lean_params;
+    l.srcp[0] = src0;
+    l.srcp[1] = src1;
+    l.initp = init;
+    l.outp = outp;
+    cudaError_t e = pmlb::launch_contract_lean(l, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return cuda_fail(e, "contract launch");
+    return PMLB_OK;
+  }
+  pmlb::GenericParams p = g;
   p.srcp[0] = src0;
   p.srcp[1] = src1;
   p.srcp[2] = src2;
   p.initp = init;
   p.outp = outp;
-  if (!outp || !src0 || (p.n_src > 1 && !src1) || (p.n_src > 2 && !src2) || (p.has_init && !init)) {
-    return fail(PMLB_ERR_INVALID, "contract: null tensor");
-  }
   cudaError_t e = pmlb::launch_contract(p, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "contract launch");
   return PMLB_OK;

@@ -443,3 +443,79 @@ def test_eltwise_dense_f32_with_bias_and_column_operands():
         outs = Runner(Program("bcast", [X, Y], [X + Y, X * Y, Y - X, X / Y]), "cuda.0").run([x, y])
         for got, want in zip(outs, (x + y, x * y, y - x, x / y)):
             np.testing.assert_array_equal(got.view(np.uint32), want.astype(np.float32).view(np.uint32), err_msg=f"{big} {small}")
+
+
+# --- the strided form of the general contraction (lean kernels) ---------------------------------------------------------
+
+def strided_case(seed):
+    """A windowed contraction with strides, dilation, padding, mirrored taps, a constraint or an initial value now and
+    then; every aggregation and combination, depthwise or with its own output channels."""
+    g = rng(7000 + seed)
+    pick = lambda *xs: xs[int(g.integers(0, len(xs)))]
+    dt = pick(K.F32, K.F32, K.F64, K.I32, K.I8)
+    n, h, w, c, co = 1 + int(g.integers(0, 2)), *(int(v) for v in g.integers(3, 9, 2)), pick(1, 3, 4, 5, 8), pick(1, 4, 6)
+    r, s, p, q = (int(v) for v in (*g.integers(1, 4, 2), *g.integers(1, 8, 2)))
+    st, dl, pd = g.integers(1, 3, 2), g.integers(1, 3, 2), g.integers(-1, 3, 2)
+    mirror = seed % 2
+    d = K.ContractDesc()
+    d.agg = pick(K.AGG_SUM, K.AGG_SUM, K.AGG_MAX, K.AGG_MIN, K.AGG_PROD, K.AGG_ASSIGN)
+    d.combo = pick(K.COMBO_MUL, K.COMBO_MUL, K.COMBO_ADD, K.COMBO_NONE)
+    d.n_src = 1 if d.combo == K.COMBO_NONE else 2
+    N, Y, X, C, I, J, CI = range(7)
+    depthwise = seed % 3 != 0
+    ranges = [n, p, q, c, r, s] if depthwise else [n, p, q, co, r, s, c]
+    d.n_idx = len(ranges)
+    for i, v in enumerate(ranges):
+        d.range[i] = v
+    shape = (n, p, q, ranges[3])
+    d.out = K.make_access(dt, shape, [{N: 1}, {Y: 1}, {X: 1}, {C: 1}])
+    rows = {Y: int(st[0]), I: int(-dl[0] if mirror else dl[0])}
+    d.src[0] = K.make_access(dt, [n, h, w, c], [{N: 1}, rows, {X: int(st[1]), J: int(dl[1])}, {C if depthwise else CI: 1}],
+                             offs=[0, int(-pd[0] + mirror * dl[0] * (r - 1)), int(-pd[1]), 0])
+    taps = (r, s, c) if depthwise else (r, s, c, co)
+    d.src[1] = K.make_access(dt, taps, [{I: 1}, {J: 1}, {C: 1}] if depthwise else [{I: 1}, {J: 1}, {CI: 1}, {C: 1}])
+    if seed % 4 == 0:
+        d.n_cons, d.cons_coef[0][I], d.cons_coef[0][X], d.cons_off[0], d.cons_range[0] = 1, 1, 1, -1, 4
+    draw = lambda sh: (g.standard_normal(sh) * (40 if dt == K.I8 else 3)).astype(NP_OF[dt])
+    init = None
+    if seed % 5 == 0:
+        d.has_init, init = 1, draw(shape[-1:])
+        d.init = K.make_access(dt, shape, None, strides=[0, 0, 0, 1])
+    return d, [draw((n, h, w, c)), draw(taps)][:d.n_src], shape, dt, init
+
+
+@pytest.mark.parametrize("seed", range(48))
+def test_strided_contraction_equals_the_walker(seed):
+    d, srcs, shape, dt, init = strided_case(seed)
+    out, ref = run_contract(d, srcs, shape, dt, init)
+    np.testing.assert_array_equal(out, ref)   # same terms, same order, every operation rounded on its own
+
+
+@pytest.mark.parametrize("n,hw,c,r,stride,dil,pad,per_channel,swap", [
+    (23, 33, 52, 3, 1, 1, 1, True, False),      # quads; runs end inside a row (33 = 8 * 4 + 1)
+    (23, 33, 51, 3, 1, 1, 1, True, True),       # single elements, filter as the first operand
+    (60, 40, 56, 3, 2, 1, 1, True, False),      # neighbours two columns apart: no shared elements
+    (33, 30, 48, 2, 1, 2, 0, True, False),      # dilation 2 against stride 1
+    (75, 31, 64, 4, 2, 2, 3, True, False),      # stride equal to the dilation, padding beyond the first tap
+    (23, 33, 52, 3, 1, 1, 1, False, False),     # one filter for all channels
+])
+def test_runs_of_neighbours_in_one_thread(n, hw, c, r, stride, dil, pad, per_channel, swap):
+    g = rng(7100 + hw + c)
+    p = (hw + 2 * pad - dil * (r - 1) - 1) // stride + 1
+    N, Y, X, C, I, J = range(6)
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 6, 2
+    for i, v in enumerate([n, p, p, c, r, r]):
+        d.range[i] = v
+    assert n * p * -(-p // 4) * (c // 4 if c % 4 == 0 else c) >= 75776   # wide enough for the kernel in question
+    d.out = K.make_access(K.F32, [n, p, p, c], [{N: 1}, {Y: 1}, {X: 1}, {C: 1}])
+    x_acc = K.make_access(K.F32, [n, hw, hw, c], [{N: 1}, {Y: stride, I: dil}, {X: stride, J: dil}, {C: 1}], offs=[0, -pad, -pad, 0])
+    f_shape = (r, r, c) if per_channel else (r, r)
+    f_acc = K.make_access(K.F32, f_shape, [{I: 1}, {J: 1}, {C: 1}][:len(f_shape)])
+    x, f = g.standard_normal((n, hw, hw, c)).astype(np.float32), g.standard_normal(f_shape).astype(np.float32)
+    d.src[0], d.src[1] = (f_acc, x_acc) if swap else (x_acc, f_acc)
+    out, ref = run_contract(d, [f, x] if swap else [x, f], (n, p, p, c), K.F32)
+    # r * r terms added in the same order, one rounding per term here and two in the walker: each at most 2^-24 of a
+    # partial sum, which stays below the sum of the terms' magnitudes
+    bound = 3 * r * r * 2.0 ** -24 * np.abs(f).max() * np.abs(x).max() * r * r
+    assert np.max(np.abs(out - ref)) <= bound
