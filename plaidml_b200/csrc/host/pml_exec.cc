@@ -1387,6 +1387,7 @@ class Planner {
     }
     pmlb_plan* plan = nullptr;
     pmlbCheck(pmlb_contract_dispatch(&d, &plan), "general contraction dispatch for '" + op.label + "'");
+    pmlbCheck(pmlb_plan_share_status(plan, exe_->status_), "status word");
     Step st;
     st.plan = plan;
     st.kernel = "generic_contract";

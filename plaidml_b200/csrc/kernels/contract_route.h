@@ -1,14 +1,112 @@
-// Which contractions leave the general kernel for the strided form of the lean kernels.  Host side only; the rule looks
-// at the descriptor alone.
+// Which contractions leave the general kernel: matrix products for the tensor cores, and the strided form of the lean
+// kernel.  Host side only; both rules look at the descriptor alone.
 #pragma once
 
 #include <stdint.h>
 
+#include <algorithm>
+#include <climits>
 #include <cstring>
+#include <vector>
 
 #include "generic.h"
 
 namespace pmlb {
+
+// A contraction as batch x (m x k times k x n) with the strides of every role in elements.
+struct ProductForm {
+  long long batch = 1, m = 1, n = 1, k = 1;
+  int a = 0, b = 1;              // sources in the roles of A and B
+  long long am = 0, ak = 0, bk = 0, bn = 0, cm = 0;   // A(i, k), B(k, j), C(i, j): C's columns are contiguous
+  long long ab = 0, bb = 0, cb = 0;                   // between batch entries
+};
+
+// Sum of products of two f32 tensors into f32 whose index expressions are single variables: every variable is a row
+// (output and one source), a column (output and the other), a term (both sources) or a batch index (all three).  The
+// variables of a role must merge into one dimension; A and B each need a contiguous dimension, the output contiguous
+// columns (exchanging the sources transposes the product).  Every output element must be reached and every read in
+// range, since the tensor-core kernel tests neither.  More than 32768 multiply-adds: up to there the lean kernel adds the
+// terms one by one in f32, which small exact expectations rely on (the planner draws the same line for its GEMMs).  With
+// A transposed, general kernel -> tensor cores: 4096 x 512 x 512 23.4 ms -> 25 us, 128 x 64 x 64 295 -> 8 us (lean kernel
+// 32 us); error against 64 bits at 4096 terms 1.1e-6 -> 2.8e-7.
+inline bool product_form(const GenericParams& p, ProductForm* out) {
+  if (p.agg != PMLB_AGG_SUM || p.combo != PMLB_COMBO_MUL || p.n_src != 2 || p.n_cons != 0 || p.has_init) return false;
+  if (p.out.dtype != PMLB_F32 || p.src[0].dtype != PMLB_F32 || p.src[1].dtype != PMLB_F32) return false;
+  const GAccess* t[3] = {&p.out, &p.src[0], &p.src[1]};
+  long long stride[3][PMLB_MAX_IDX];
+  bool has[3][PMLB_MAX_IDX];
+  double macs = 1;
+  for (int i = 0; i < p.n_idx; ++i) {
+    if (p.range[i] <= 0) return false;
+    macs *= static_cast<double>(p.range[i]);
+    for (int s = 0; s < 3; ++s) has[s][i] = false, stride[s][i] = 0;
+  }
+  if (macs <= 32768.0) return false;
+  for (int s = 0; s < 3; ++s) {
+    for (int d = 0; d < t[s]->rank; ++d) {
+      if (t[s]->off[d] != 0 || t[s]->den[d] != 1 || t[s]->strides[d] < 0) return false;
+      int var = -1;
+      for (int i = 0; i < p.n_idx; ++i) {
+        if (t[s]->coef[d][i] == 0 || p.range[i] == 1) continue;   // (a single-valued variable is 0)
+        if (var >= 0 || t[s]->coef[d][i] != 1) return false;
+        var = i;
+      }
+      if (var < 0) {
+        if (t[s]->sizes[d] < 1 || (s == 0 && t[s]->sizes[d] != 1)) return false;
+        continue;
+      }
+      if (has[s][var]) return false;   // a diagonal
+      if (s == 0 ? p.range[var] != t[s]->sizes[d] : p.range[var] > t[s]->sizes[d]) return false;
+      has[s][var] = true;
+      stride[s][var] = t[s]->strides[d];
+    }
+  }
+  for (int order = 0; order < 2; ++order) {
+    const int sa = 1 + order, sb = 2 - order;
+    struct Role {
+      std::vector<int> vars;
+      long long extent = 1, so = 0, sa = 0, sb = 0;
+    } m, n, k, b;
+    bool ok = true;
+    for (int i = 0; i < p.n_idx && ok; ++i) {
+      if (p.range[i] == 1) continue;
+      const bool o = has[0][i], x = has[sa][i], y = has[sb][i];
+      if (o && x && y) b.vars.push_back(i);
+      else if (o && x) m.vars.push_back(i);
+      else if (o && y) n.vars.push_back(i);
+      else if (x && y) k.vars.push_back(i);
+      else ok = false;
+    }
+    auto merge = [&](Role* r, int key) {
+      std::sort(r->vars.begin(), r->vars.end(), [&](int x, int y) { return stride[key][x] > stride[key][y]; });
+      for (size_t j = 0; j < r->vars.size(); ++j) {
+        const int v = r->vars[j];
+        r->extent *= p.range[v];
+        if (j + 1 == r->vars.size()) {
+          r->so = stride[0][v], r->sa = stride[sa][v], r->sb = stride[sb][v];
+        } else {
+          const int w = r->vars[j + 1];
+          for (int s = 0; s < 3; ++s) {
+            if (has[s][v] && stride[s][v] != stride[s][w] * p.range[w]) return false;
+          }
+        }
+      }
+      return true;
+    };
+    ok = ok && merge(&m, 0) && merge(&n, 0) && merge(&b, 0) && merge(&k, sa);
+    if (!ok || m.extent > INT_MAX || n.extent > INT_MAX || k.extent > INT_MAX || b.extent > INT_MAX) continue;
+    if (n.extent > 1 && n.so != 1) continue;
+    if (m.extent > 1 && n.extent > 1 && m.so < n.extent) continue;
+    if (m.extent > 1 && m.sa != 1 && k.extent > 1 && k.sa != 1) continue;
+    if (n.extent > 1 && n.sb != 1 && k.extent > 1 && k.sb != 1) continue;
+    out->batch = b.extent, out->m = m.extent, out->n = n.extent, out->k = k.extent;
+    out->a = sa - 1, out->b = sb - 1;
+    out->am = m.sa, out->ak = k.sa, out->bk = k.sb, out->bn = n.sb, out->cm = m.so;
+    out->ab = b.sa, out->bb = b.sb, out->cb = b.so;
+    return true;
+  }
+  return false;
+}
 
 // The lean kernel's form: see generic.cu.  Output dims are single variables without offset, everything is integral,
 // offsets fit 32 bits, at most four of the variables that are not in the output have a range above 1, and at most four

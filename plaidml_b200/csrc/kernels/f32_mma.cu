@@ -765,9 +765,9 @@ struct Choice {
 // reads, the loaders' stores and the loads share the SM's 128 bytes per cycle) and 3750 on a CTA pair for four times
 // the 128-wide tile's work on two SMs (the rate the tensor pipe sustains); rows that are not 16-byte aligned cost a
 // third more loads.  Everything around the loop: 8800, 11500 and 18000 cycles, and 1500 + 150 per CTA of a K split.
-Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_override, int split_override, int dev, int sms) {
+Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_override, int split_override, bool pairs, int dev, int sms) {
   Choice best;
-  for (int bn = 64; bn <= 256; bn *= 2) {
+  for (int bn = 64; bn <= (pairs ? 256 : 128); bn *= 2) {
     if (bn_override != 0 && bn != bn_override) continue;
     const int rows = bn == 256 ? 256 : 128;
     const long long tiles = static_cast<long long>((m + rows - 1) / rows) * ((n + bn - 1) / bn) * batch;
@@ -821,7 +821,7 @@ bool f32_mma_faster(const F32MmaShape& s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, dev, sms);
+  const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, true, dev, sms);
   const double here = c.cycles / 1900.0 * (s.conv ? 1.2 : 1.0);
   const double tiles_m = (s.m + 127) / 128;
   auto prepass = [&](int bn, double block_us) {
@@ -862,7 +862,7 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const Choice best = choose_tiles(L.m, L.n, p.num_kb, L.batch, vec, L.bn_override, L.split_override, dev, sms);
+  const Choice best = choose_tiles(L.m, L.n, p.num_kb, L.batch, vec, L.bn_override, L.split_override, !L.short_chains, dev, sms);
   const int best_bn = best.bn, best_split = best.split;
   if (best_bn == 0) {
     *err = "no tile fits the requested K split";

@@ -29,6 +29,7 @@ struct F32MmaLaunch {
   float* rowmax = nullptr;          // f32[batch * m], filled with -inf by the caller
   int* status = nullptr;            // device word that receives a non-zero code if a wait times out
   int bn_override = 0;              // 0 = choose; else 64, 128 or 256
+  bool short_chains = false;        // no CTA pairs, whose accumulator chains run over all of K
   int split_override = 0;           // 0 = choose; else the number of CTAs (1..8) that share a tile's K range
 };
 

@@ -117,8 +117,9 @@ struct pmlb_plan {
   pmlb_reduce_desc reduce;
   pmlb_pool_desc pool;
   pmlb::GenericParams generic;
-  bool lean = false;             // contraction: strided form (else the general kernel)
+  bool lean = false;             // contraction: strided form (else the general kernel, or f32_mma)
   pmlb::LeanParams lean_params;
+  pmlb::ProductForm product;     // contraction on the tensor cores (f32_mma)
   pmlb::EltwiseParams eltwise;
   pmlb_special_desc special;
 };
@@ -1079,8 +1080,13 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
       if (!direct || !used[i]) p.loop_var[p.n_loop++] = i;
     }
   }
-  plan->lean = pmlb::lean_form(p, &plan->lean_params);
-  cudaGetDevice(&plan->device);
+  plan->f32_mma = pmlb::product_form(p, &plan->product);
+  plan->lean = !plan->f32_mma && pmlb::lean_form(p, &plan->lean_params);
+  pmlb_status st = alloc_plan_memory(plan, 0, plan->f32_mma);
+  if (st != PMLB_OK) {
+    pmlb_plan_free(plan);
+    return st;
+  }
   *out = plan;
   return PMLB_OK;
 }
@@ -1091,6 +1097,25 @@ pmlb_status pmlb_contract_invoke(pmlb_plan* plan, void* stream, const void* src0
   const pmlb::GenericParams& g = plan->generic;
   if (!outp || !src0 || (g.n_src > 1 && !src1) || (g.n_src > 2 && !src2) || (g.has_init && !init)) {
     return fail(PMLB_ERR_INVALID, "contract: null tensor");
+  }
+  if (plan->f32_mma) {
+    const pmlb::ProductForm& f = plan->product;
+    const void* src[2] = {src0, src1};
+    pmlb::F32MmaLaunch L;
+    L.m = static_cast<int>(f.m), L.n = static_cast<int>(f.n), L.k = static_cast<int>(f.k), L.batch = static_cast<int>(f.batch);
+    L.a = static_cast<const float*>(src[f.a]), L.a_batch = f.ab;
+    L.a_mn = f.k > 1 && f.ak != 1;
+    L.lda = L.a_mn ? f.ak : f.am;
+    L.b = static_cast<const float*>(src[f.b]), L.b_batch = f.bb;
+    L.b_mn = f.k > 1 && f.bk != 1;
+    L.ldb = L.b_mn ? f.bk : f.bn;
+    L.out = static_cast<float*>(outp), L.ldc = f.cm, L.out_batch = f.cb;
+    L.status = plan->status;
+    L.short_chains = true;
+    std::string err;
+    const int rc = pmlb::f32_mma_launch(L, static_cast<cudaStream_t>(stream), &err);
+    if (rc != 0) return fail(static_cast<pmlb_status>(rc), "contract: " + err);
+    return PMLB_OK;
   }
   if (plan->lean) {
     pmlb::LeanParams l = plan->lean_params;

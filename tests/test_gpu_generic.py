@@ -445,7 +445,7 @@ def test_eltwise_dense_f32_with_bias_and_column_operands():
             np.testing.assert_array_equal(got.view(np.uint32), want.astype(np.float32).view(np.uint32), err_msg=f"{big} {small}")
 
 
-# --- the strided form of the general contraction (lean kernels) ---------------------------------------------------------
+# --- the strided form (lean kernels) and matrix products of the general contraction -----------------------------------
 
 def strided_case(seed):
     """A windowed contraction with strides, dilation, padding, mirrored taps, a constraint or an initial value now and
@@ -519,3 +519,43 @@ def test_runs_of_neighbours_in_one_thread(n, hw, c, r, stride, dil, pad, per_cha
     # partial sum, which stays below the sum of the terms' magnitudes
     bound = 3 * r * r * 2.0 ** -24 * np.abs(f).max() * np.abs(x).max() * r * r
     assert np.max(np.abs(out - ref)) <= bound
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_products_in_any_order_of_dims(seed):
+    # every order of the dims of both operands and of the result: transposed operands, batch dims outside or inside,
+    # orders that no single matrix product covers (these stay with the strided form)
+    g = rng(7200 + seed)
+    ext = {"m": int(g.integers(1, 150)), "n": int(g.integers(1, 150)), "k": int(g.integers(1, 300)), "b": int(g.integers(1, 4))}
+    while ext["m"] * ext["n"] * ext["k"] * ext["b"] <= 32768:
+        ext["k"] = 2 * ext["k"] + 1
+    var = {v: i for i, v in enumerate("mnkb")}
+    a, b, c = ("".join(g.permutation(list(v))) for v in ("mkb", "knb", "mnb"))
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 4, 2
+    for v, i in var.items():
+        d.range[i] = ext[v]
+    acc = lambda dims: K.make_access(K.F32, [ext[v] for v in dims], [{var[v]: 1} for v in dims])
+    d.out, d.src[0], d.src[1] = acc(c), acc(a), acc(b)
+    x, y = (g.standard_normal([ext[v] for v in dims]).astype(np.float32) for dims in (a, b))
+    out, ref = run_contract(d, [x, y], tuple(ext[v] for v in c), K.F32)
+    want = np.einsum(f"{a},{b}->{c}", x.astype(np.float64), y.astype(np.float64))
+    norm = np.linalg.norm(want)
+    # no further from the exact sums than the one-by-one f32 sums, or than 2^-20 where there are few terms
+    assert np.linalg.norm(out - want) / norm <= max(1.5 * np.linalg.norm(ref - want) / norm, 2.0 ** -20)
+
+
+def test_product_that_does_not_cover_its_output_or_reads_out_of_range_stays_exact():
+    # a range shorter than the output dim leaves the identity there; one longer than an operand's dim skips terms
+    g = rng(7300)
+    a, b = g.standard_normal((64, 50)).astype(np.float32), g.standard_normal((64, 60)).astype(np.float32)
+    for m, k, rows in ((40, 64, 50), (50, 70, 50)):
+        d = K.ContractDesc()
+        d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 3, 2
+        for i, v in enumerate([m, 60, k]):
+            d.range[i] = v
+        d.out = K.make_access(K.F32, [rows, 60], [{0: 1}, {1: 1}])
+        d.src[0] = K.make_access(K.F32, [64, 50], [{2: 1}, {0: 1}])
+        d.src[1] = K.make_access(K.F32, [64, 60], [{2: 1}, {1: 1}])
+        out, ref = run_contract(d, [a, b], (rows, 60), K.F32)
+        np.testing.assert_array_equal(out, ref)
