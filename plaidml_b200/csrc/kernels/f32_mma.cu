@@ -37,6 +37,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "pmlb_kernels.h"
@@ -719,12 +720,16 @@ __global__ void __launch_bounds__(256) filter_to_f32_kernel(const In* in, float*
 
 using KernelPtr = void (*)(const F32MmaParams);
 
+// The shared-memory limit is an attribute per device.
 template <int BN, int AL, int BL, bool VEC>
-KernelPtr instance() {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(f32_mma_kernel<BN, AL, BL, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Cfg<BN>::kSmem);
-  });
+KernelPtr instance(int dev) {
+  static std::atomic<uint64_t> done{0};
+  const uint64_t bit = 1ull << (dev & 63);
+  if (dev >= 64 || (done.load(std::memory_order_acquire) & bit) == 0) {
+    if (cudaFuncSetAttribute(f32_mma_kernel<BN, AL, BL, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Cfg<BN>::kSmem) == cudaSuccess) {
+      done.fetch_or(bit, std::memory_order_release);
+    }
+  }
   return f32_mma_kernel<BN, AL, BL, VEC>;
 }
 
@@ -746,7 +751,7 @@ int resident_clusters(int dev, int split) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, instance<64, kRowsK, kRowsMn, true>(), &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, instance<64, kRowsK, kRowsMn, true>(dev), &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = 1;
     }
@@ -790,14 +795,14 @@ Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_overri
 }
 
 template <int BN>
-KernelPtr choose(int al, int bl, bool vec) {
-  if (al == kRowsConv) return vec ? instance<BN, kRowsConv, kRowsMn, true>() : instance<BN, kRowsConv, kRowsMn, false>();
+KernelPtr choose(int al, int bl, bool vec, int dev) {
+  if (al == kRowsConv) return vec ? instance<BN, kRowsConv, kRowsMn, true>(dev) : instance<BN, kRowsConv, kRowsMn, false>(dev);
   if (vec) {
-    if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, true>() : instance<BN, kRowsK, kRowsMn, true>();
-    return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, true>() : instance<BN, kRowsMn, kRowsMn, true>();
+    if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, true>(dev) : instance<BN, kRowsK, kRowsMn, true>(dev);
+    return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, true>(dev) : instance<BN, kRowsMn, kRowsMn, true>(dev);
   }
-  if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, false>() : instance<BN, kRowsK, kRowsMn, false>();
-  return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, false>() : instance<BN, kRowsMn, kRowsMn, false>();
+  if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, false>(dev) : instance<BN, kRowsK, kRowsMn, false>(dev);
+  return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, false>(dev) : instance<BN, kRowsMn, kRowsMn, false>(dev);
 }
 
 }  // namespace
@@ -811,18 +816,29 @@ bool f32_mma_takes_conv(const ConvGeom& g) {
          static_cast<long long>(g.n) * g.p * g.q < (1ll << 30) && static_cast<long long>(g.r) * g.s * g.c < (1ll << 30);
 }
 
+F32MmaTiles f32_mma_tiles(const F32MmaShape& s) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, s.tile_n, s.whole_k ? 1 : 0, !s.short_chains, dev, sms);
+  F32MmaTiles t;
+  t.bn = c.bn, t.split = c.split;
+  return t;
+}
+
 // Both estimates in microseconds.  The pre-pass route (B200, graph replays): 9 us of launches and set-up, 12 bytes per
 // element at 5.2 TB/s, then 0.58 (128-wide tiles) or 0.38 us (64-wide) per 32 terms of each wave of a persistent grid
 // that stores one tile while it computes the next, a third more where rows are not 16-byte aligned.  It wins where a
 // launch has several waves of tiles and each of them few terms, because this file's kernel stores a tile before its SM
 // starts the next: 4096 x 4096 x 256 46 against 71 us, 100352 x 64 x 576 72 against 93 us; it loses on few tiles, long
 // K, odd rows and strided 1x1 convolutions: 64 x 4096 x 4096 94 against 29 us, 1999 x 2001 x 1001 70 against 55 us.
-bool f32_mma_faster(const F32MmaShape& s) {
+bool f32_mma_faster(const F32MmaShape& s, F32MmaTiles* tiles) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, true, dev, sms);
-  const double here = c.cycles / 1900.0 * (s.conv ? 1.2 : 1.0);
+  const Choice any = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, true, dev, sms);
+  const double here = any.cycles / 1900.0 * (s.conv ? 1.2 : 1.0);
+  *tiles = f32_mma_tiles(s);
   const double tiles_m = (s.m + 127) / 128;
   auto prepass = [&](int bn, double block_us) {
     const double waves = std::max(1.0, tiles_m * ((s.n + bn - 1) / bn) * s.batch / sms);
@@ -859,16 +875,10 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
     p.fd_pq = make_fastdiv(g.p * g.q);
     p.fd_q = make_fastdiv(g.q);
   }
-  int dev = 0, sms = 0;
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const Choice best = choose_tiles(L.m, L.n, p.num_kb, L.batch, vec, L.bn_override, L.split_override, !L.short_chains, dev, sms);
-  const int best_bn = best.bn, best_split = best.split;
-  if (best_bn == 0) {
-    *err = "no tile fits the requested K split";
-    return PMLB_ERR_INVALID;
-  }
-  p.split = best_split;
+  const int best_bn = L.tiles.bn;
+  p.split = L.tiles.split;
   p.tiles_n = (L.n + best_bn - 1) / best_bn;
   const int tile_rows = best_bn == 256 ? 256 : 128, share = best_bn == 256 ? 2 : p.split;
   const long long per_batch = static_cast<long long>((L.m + tile_rows - 1) / tile_rows) * p.tiles_n;
@@ -880,7 +890,7 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   p.tiles_per_batch = static_cast<int>(per_batch);
   const long long grid = units * share;
   const int bl = L.b_mn ? kRowsMn : kRowsK;
-  const KernelPtr kernel = best_bn == 256 ? choose<256>(al, bl, vec) : (best_bn == 128 ? choose<128>(al, bl, vec) : choose<64>(al, bl, vec));
+  const KernelPtr kernel = best_bn == 256 ? choose<256>(al, bl, vec, dev) : (best_bn == 128 ? choose<128>(al, bl, vec, dev) : choose<64>(al, bl, vec, dev));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kThreads);

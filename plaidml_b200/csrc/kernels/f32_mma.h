@@ -9,6 +9,11 @@
 
 namespace pmlb {
 
+// Tile width (64, 128: one CTA; 256: a CTA pair) and the number of CTAs (1..8) that share a tile's K range.
+struct F32MmaTiles {
+  int bn = 64, split = 1;
+};
+
 // C[b][i][j] = sum_k A(b, i, k) * B(b, k, j), everything fp32 in device memory.
 struct F32MmaLaunch {
   int m = 0, n = 0, k = 0, batch = 1;
@@ -28,22 +33,27 @@ struct F32MmaLaunch {
   long long ldr = 0, res_batch = 0;
   float* rowmax = nullptr;          // f32[batch * m], filled with -inf by the caller
   int* status = nullptr;            // device word that receives a non-zero code if a wait times out
-  int bn_override = 0;              // 0 = choose; else 64, 128 or 256
-  bool short_chains = false;        // no CTA pairs, whose accumulator chains run over all of K
-  int split_override = 0;           // 0 = choose; else the number of CTAs (1..8) that share a tile's K range
+  F32MmaTiles tiles;
 };
 
 // Whether the kernel accepts a convolution.
 bool f32_mma_takes_conv(const ConvGeom& g);
 
-// Whether the kernel is expected to be faster than splitting the operands into TF32 parts by pre-passes.
 struct F32MmaShape {
   int m = 0, n = 0, k = 0, batch = 1;
   bool conv = false;
   bool aligned_in = true, aligned_out = true;   // rows start on 16-byte boundaries
   long long elems = 0;                          // elements that each call's pre-pass would split
+  int tile_n = 0;                               // 0 = choose; else 64 or 128
+  bool whole_k = false;                         // no K split
+  bool short_chains = false;                    // no CTA pairs, whose accumulator chains run over all of K
 };
-bool f32_mma_faster(const F32MmaShape& shape);
+
+// The tiles a shape is expected to run fastest with.
+F32MmaTiles f32_mma_tiles(const F32MmaShape& shape);
+
+// Whether the kernel is expected to be faster than splitting the operands into TF32 parts by pre-passes, and its tiles.
+bool f32_mma_faster(const F32MmaShape& shape, F32MmaTiles* tiles);
 
 // Returns 0 on success, otherwise a pmlb_status value with a message in *err.
 int f32_mma_launch(const F32MmaLaunch& launch, cudaStream_t stream, std::string* err);

@@ -100,9 +100,9 @@ struct pmlb_plan {
   long long kpad = 0;       // transposed B, split fp32 operands: padded K or channel count
   bool transpose_b = false; // 8/16-bit path: B goes through [n][k] scratch
   bool f32_mma = false;     // fp32 operands split inside the kernel (f32_mma.cu)
+  pmlb::F32MmaTiles f32_tiles;
   bool split = false;       // fp32 operands split into TF32 parts by pre-passes
   int armed_wait_us = 0;    // > 0: the next invoke runs the time-out test (see pmlb_plan_arm_timeout_test)
-  bool ksplit_off = false;  // the caller (or the environment) wants K in one part
   int ksplit = 1;           // parts of the K range (two-pass split-K), each of kslice elements
   long long kslice = 0;
 
@@ -342,8 +342,11 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
     shape.aligned_in = d->lda % 4 == 0 && d->ldb % 4 == 0;
     shape.aligned_out = d->ldc % 4 == 0;
     shape.elems = (a_mats * d->m + b_mats * d->n) * d->k;
+    shape.tile_n = d->tile_n;
+    const char* env = std::getenv("PMLB_SPLIT_K");
+    shape.whole_k = (d->flags & PMLB_GEMM_NO_SPLIT_K) != 0 || (env && env[0] == '0');
     // (a forced 256-wide tile is refused for f32, by the other route)
-    if ((d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_faster(shape)) {
+    if ((d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_faster(shape, &plan->f32_tiles)) {
       plan->f32_mma = true;   // no scratch but the status word
       scratch = 256;
     } else {
@@ -371,7 +374,6 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
   // Split K?  (8/16-bit inputs read in place, one matrix, no row maxima: see PMLB_GEMM_NO_SPLIT_K)
   const char* split_env = std::getenv("PMLB_SPLIT_K");   // "0": never split (sums then never depend on the tile count)
   const bool split_allowed = !(split_env && split_env[0] == '0') || (d->flags & PMLB_GEMM_SPLIT_K);
-  plan->ksplit_off = !split_allowed || (d->flags & PMLB_GEMM_NO_SPLIT_K) != 0;
   if (!f32 && !plan->transpose_b && d->batch == 1 && !(d->epilogue & PMLB_EPI_ROWMAX) && d->k_first == 0 &&
       !(d->flags & PMLB_GEMM_NO_SPLIT_K) && split_allowed) {
     const int bk = 128 / eb;
@@ -445,8 +447,7 @@ pmlb_status pmlb_gemm_invoke_two(pmlb_plan* plan, void* stream_v, const void* a,
     f.ldr = d.ldr, f.res_batch = d.stride_r;
     f.rowmax = rowmax;
     f.status = plan->status;
-    f.bn_override = d.tile_n;
-    if (plan->ksplit_off) f.split_override = 1;
+    f.tiles = plan->f32_tiles;
     if (d.epilogue & PMLB_EPI_ROWMAX) {
       cudaError_t e = pmlb::launch_fill_f32(rowmax, static_cast<long long>(d.batch) * d.m, -__builtin_inff(), stream);
       if (e != cudaSuccess) return cuda_fail(e, "fill(rowmax)");
@@ -639,9 +640,12 @@ pmlb_status pmlb_conv_dispatch(const pmlb_conv_desc* d, pmlb_plan** out) {
   shape.conv = true;
   shape.aligned_in = shape.aligned_out = d->k % 4 == 0;
   shape.elems = static_cast<long long>(d->n) * d->h * d->w * d->c;
+  shape.tile_n = d->tile_n;
+  pmlb::F32MmaTiles f32_tiles;
   if (f32 && (d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_takes_conv(conv_geom(*d)) &&
-      pmlb::f32_mma_faster(shape)) {
+      pmlb::f32_mma_faster(shape, &f32_tiles)) {
     plan->f32_mma = true;
+    plan->f32_tiles = f32_tiles;
     scratch = static_cast<size_t>(d->k) * d->r * d->s * d->c * 4;   // the filter, [r][s][c][k] in f32
   } else if (f32) {
     // fp32: three TF32 products per term (as the fp32 GEMM): the filter and, per call, the activation are split
@@ -840,7 +844,7 @@ pmlb_status pmlb_conv_invoke(pmlb_plan* plan, void* stream, const void* input, v
     f.residual = (d.epilogue & PMLB_EPI_RESIDUAL) ? static_cast<const float*>(residual) : nullptr;
     f.ldr = d.k;
     f.status = plan->status;
-    f.bn_override = d.tile_n;
+    f.tiles = plan->f32_tiles;
     std::string err;
     const int rc = pmlb::f32_mma_launch(f, static_cast<cudaStream_t>(stream), &err);
     if (rc != 0) return fail(static_cast<pmlb_status>(rc), "conv: " + err);
@@ -1082,6 +1086,14 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
   }
   plan->f32_mma = pmlb::product_form(p, &plan->product);
   plan->lean = !plan->f32_mma && pmlb::lean_form(p, &plan->lean_params);
+  if (plan->f32_mma) {
+    const pmlb::ProductForm& f = plan->product;
+    pmlb::F32MmaShape shape;
+    shape.m = static_cast<int>(f.m), shape.n = static_cast<int>(f.n), shape.k = static_cast<int>(f.k), shape.batch = static_cast<int>(f.batch);
+    shape.aligned_in = (f.ak == 1 ? f.am : f.ak) % 4 == 0 && (f.bk == 1 ? f.bn : f.bk) % 4 == 0;
+    shape.short_chains = true;
+    plan->f32_tiles = pmlb::f32_mma_tiles(shape);
+  }
   pmlb_status st = alloc_plan_memory(plan, 0, plan->f32_mma);
   if (st != PMLB_OK) {
     pmlb_plan_free(plan);
@@ -1111,7 +1123,7 @@ pmlb_status pmlb_contract_invoke(pmlb_plan* plan, void* stream, const void* src0
     L.ldb = L.b_mn ? f.bk : f.bn;
     L.out = static_cast<float*>(outp), L.ldc = f.cm, L.out_batch = f.cb;
     L.status = plan->status;
-    L.short_chains = true;
+    L.tiles = plan->f32_tiles;
     std::string err;
     const int rc = pmlb::f32_mma_launch(L, static_cast<cudaStream_t>(stream), &err);
     if (rc != 0) return fail(static_cast<pmlb_status>(rc), "contract: " + err);
