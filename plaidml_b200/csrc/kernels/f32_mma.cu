@@ -41,6 +41,7 @@
 #include <mutex>
 
 #include "pmlb_kernels.h"
+#include "dependent_launch.h"
 #include "ptx.cuh"
 #include "tc_gemm.cuh"
 
@@ -452,6 +453,8 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
       la.origin = p.a + batch * p.a_batch + (AL == kRowsMn ? static_cast<long long>(m0) : static_cast<long long>(m0) * p.lda);
     }
     lb.origin = p.b + batch * p.b_batch + (BL == kRowsMn ? static_cast<long long>(nb0) : static_cast<long long>(nb0) * p.ldb);
+    grid_dependency_wait();
+    grid_launch_dependents();
     // (the first loads are on their way while the barriers and TMEM are set up)
     la.load(kb_begin * kBlockK, p, tid);
     lb.load(kb_begin * kBlockK, p, tid);
@@ -652,6 +655,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
     __syncthreads();
   }
   const bool failed = abort_flag[0] != 0;
+  grid_dependency_wait();   // (long past for the loaders; the other warps have not touched global memory yet)
   if (!failed && warp < kIssuerWarp) {
     constexpr int kPieces = BN / 4;                 // 16-byte pieces per row
     const int strip = (128 + strips - 1) / strips;
@@ -896,12 +900,13 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = best_bn == 256 ? F32Cfg<256>::kSmem : (best_bn == 128 ? F32Cfg<128>::kSmem : F32Cfg<64>::kSmem);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = share;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0] = dependent_launch_attribute();
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = share;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = share > 1 ? 1 : 0;
+  cfg.numAttrs = share > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) {
     *err = std::string("fp32 tensor-core launch: ") + cudaGetErrorString(e);

@@ -14,6 +14,7 @@
 // Arithmetic happens in the contraction's element type: integers wrap (computed in 64
 // bits and truncated on store), f16 / bf16 round after every operation, max / min are a
 // compare-and-select with an ordered compare.
+#include "dependent_launch.h"
 #include "generic.h"
 #include "typed_access.cuh"
 
@@ -70,6 +71,7 @@ __device__ __forceinline__ long long floor_div_exact(long long num, int den, boo
 
 template <class T>
 __global__ void __launch_bounds__(256) contract_kernel(const __grid_constant__ GenericParams p) {
+  dependent_entry();
   const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= p.out_elems) return;
 
@@ -303,6 +305,7 @@ __device__ __forceinline__ void lean_clip(int c, int step, int size, int* lo, in
 // 86 us, and 6 us on one image (142 us before).
 template <int V>
 __global__ void __launch_bounds__(256) contract_lean_f32_kernel(const __grid_constant__ LeanParams p) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (t * V >= p.elems) return;
   const LeanPlace w = lean_place(p, static_cast<int>(t * V));
@@ -431,6 +434,7 @@ __device__ __forceinline__ RunVec<W> run_load(const float* p) {
 template <int W, bool ONE_M, bool ONE_F, int NT>
 __global__ void __launch_bounds__(kRunBlock, 1024 / kRunBlock)
 contract_lean_run_kernel(const __grid_constant__ LeanParams p, const __grid_constant__ LeanRun r) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * kRunBlock + threadIdx.x;
   if (t >= r.threads) return;
   const int last = p.rank - 1, along = p.rank - 2;
@@ -559,6 +563,7 @@ contract_lean_run_kernel(const __grid_constant__ LeanParams p, const __grid_cons
 // The same for any element types, one element per thread, values in the class of the output type.
 template <class T>
 __global__ void __launch_bounds__(256) contract_lean_kernel(const __grid_constant__ LeanParams p) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (t >= p.elems) return;
   const LeanPlace w = lean_place(p, static_cast<int>(t));
@@ -713,6 +718,7 @@ __device__ __forceinline__ void eltwise_one(const EltwiseParams& p, long long e,
 
 template <class T>
 __global__ void __launch_bounds__(256) eltwise_kernel(const __grid_constant__ EltwiseParams p) {
+  dependent_entry();
   const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= p.elems) return;
   long long rem = e;
@@ -732,6 +738,7 @@ __global__ void __launch_bounds__(256) eltwise_kernel(const __grid_constant__ El
 template <class T>
 __global__ void __launch_bounds__(256) eltwise_dense_kernel(const __grid_constant__ EltwiseParams p, int one_value,
                                                             long long threads) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= threads) return;
 #pragma unroll
@@ -757,6 +764,7 @@ struct DenseF32 {
 };
 
 __global__ void __launch_bounds__(256) eltwise_f32_dense_kernel(const DenseF32 p, long long threads) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= threads) return;
   float4 v[2][3];
@@ -813,6 +821,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 shorten<__nv_bfloat16>(floa
 
 template <class S>
 __global__ void __launch_bounds__(256) eltwise_16bit_dense_kernel(const Dense16<S> p) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= p.octets) return;
   struct alignas(16) Vec { S v[8]; };
@@ -850,6 +859,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 convert_one<float, __nv_bfl
 
 template <class In, class Out>
 __global__ void __launch_bounds__(256) convert_dense_kernel(const In* __restrict__ in, Out* __restrict__ out, long long octets) {
+  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= octets) return;
   struct alignas(sizeof(In) * 8) InVec { In v[8]; };
@@ -863,6 +873,7 @@ __global__ void __launch_bounds__(256) convert_dense_kernel(const In* __restrict
 
 template <class T>
 __global__ void __launch_bounds__(256) fill_kernel(void* out, int dtype, long long n, T value) {
+  dependent_entry();
   const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e < n) store_as<T>(out, dtype, e, value);
 }
@@ -894,10 +905,10 @@ cudaError_t launch_contract(const GenericParams& p, cudaStream_t stream) {
   if (p.out_elems <= 0) return cudaSuccess;
   const unsigned grid = grid_for(p.out_elems);
   switch (dtype_class(p.out.dtype)) {
-    case kClassF32: contract_kernel<float><<<grid, 256, 0, stream>>>(p); break;
-    case kClassF64: contract_kernel<double><<<grid, 256, 0, stream>>>(p); break;
-    case kClassI64: contract_kernel<long long><<<grid, 256, 0, stream>>>(p); break;
-    case kClassU64: contract_kernel<unsigned long long><<<grid, 256, 0, stream>>>(p); break;
+    case kClassF32: launch_dependent(contract_kernel<float>, grid, 256, stream, p); break;
+    case kClassF64: launch_dependent(contract_kernel<double>, grid, 256, stream, p); break;
+    case kClassI64: launch_dependent(contract_kernel<long long>, grid, 256, stream, p); break;
+    case kClassU64: launch_dependent(contract_kernel<unsigned long long>, grid, 256, stream, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -937,9 +948,9 @@ template <int W, bool ONE_M, bool ONE_F>
 void launch_run(const LeanParams& p, const LeanRun& r, cudaStream_t stream) {
   const unsigned grid = static_cast<unsigned>((r.threads + kRunBlock - 1) / kRunBlock);
   if (r.n_clip <= 1 && r.n_test <= 1) {
-    contract_lean_run_kernel<W, ONE_M, ONE_F, 1><<<grid, kRunBlock, 0, stream>>>(p, r);
+    launch_dependent(contract_lean_run_kernel<W, ONE_M, ONE_F, 1>, grid, kRunBlock, stream, p, r);
   } else {
-    contract_lean_run_kernel<W, ONE_M, ONE_F, 4><<<grid, kRunBlock, 0, stream>>>(p, r);
+    launch_dependent(contract_lean_run_kernel<W, ONE_M, ONE_F, 4>, grid, kRunBlock, stream, p, r);
   }
 }
 }  // namespace
@@ -969,18 +980,18 @@ cudaError_t launch_contract_lean(const LeanParams& p, cudaStream_t stream) {
       else if (one_f) launch_run<4, false, true>(p, run, stream);
       else launch_run<4, false, false>(p, run, stream);
     } else if (quads) {
-      contract_lean_f32_kernel<4><<<grid_for(p.elems / 4), 256, 0, stream>>>(p);
+      launch_dependent(contract_lean_f32_kernel<4>, grid_for(p.elems / 4), 256, stream, p);
     } else {
-      contract_lean_f32_kernel<1><<<grid_for(p.elems), 256, 0, stream>>>(p);
+      launch_dependent(contract_lean_f32_kernel<1>, grid_for(p.elems), 256, stream, p);
     }
     return cudaGetLastError();
   }
   const unsigned grid = grid_for(p.elems);
   switch (dtype_class(p.out_dtype)) {
-    case kClassF32: contract_lean_kernel<float><<<grid, 256, 0, stream>>>(p); break;
-    case kClassF64: contract_lean_kernel<double><<<grid, 256, 0, stream>>>(p); break;
-    case kClassI64: contract_lean_kernel<long long><<<grid, 256, 0, stream>>>(p); break;
-    case kClassU64: contract_lean_kernel<unsigned long long><<<grid, 256, 0, stream>>>(p); break;
+    case kClassF32: launch_dependent(contract_lean_kernel<float>, grid, 256, stream, p); break;
+    case kClassF64: launch_dependent(contract_lean_kernel<double>, grid, 256, stream, p); break;
+    case kClassI64: launch_dependent(contract_lean_kernel<long long>, grid, 256, stream, p); break;
+    case kClassU64: launch_dependent(contract_lean_kernel<unsigned long long>, grid, 256, stream, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -1073,14 +1084,14 @@ bool launch_dense_convert(const EltwiseParams& p, cudaStream_t stream) {
   const unsigned grid = grid_for(octets);
   const int from = p.in_dtype[0], to = p.out_dtype;
   if (from == PMLB_F32 && to == PMLB_F16) {
-    convert_dense_kernel<float, __half><<<grid, 256, 0, stream>>>(static_cast<const float*>(p.in[0]), static_cast<__half*>(p.out), octets);
+    launch_dependent(convert_dense_kernel<float, __half>, grid, 256, stream, static_cast<const float*>(p.in[0]), static_cast<__half*>(p.out), octets);
   } else if (from == PMLB_F32 && to == PMLB_BF16) {
-    convert_dense_kernel<float, __nv_bfloat16><<<grid, 256, 0, stream>>>(static_cast<const float*>(p.in[0]),
+    launch_dependent(convert_dense_kernel<float, __nv_bfloat16>, grid, 256, stream, static_cast<const float*>(p.in[0]),
                                                                          static_cast<__nv_bfloat16*>(p.out), octets);
   } else if (from == PMLB_F16 && to == PMLB_F32) {
-    convert_dense_kernel<__half, float><<<grid, 256, 0, stream>>>(static_cast<const __half*>(p.in[0]), static_cast<float*>(p.out), octets);
+    launch_dependent(convert_dense_kernel<__half, float>, grid, 256, stream, static_cast<const __half*>(p.in[0]), static_cast<float*>(p.out), octets);
   } else if (from == PMLB_BF16 && to == PMLB_F32) {
-    convert_dense_kernel<__nv_bfloat16, float><<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(p.in[0]),
+    launch_dependent(convert_dense_kernel<__nv_bfloat16, float>, grid, 256, stream, static_cast<const __nv_bfloat16*>(p.in[0]),
                                                                          static_cast<float*>(p.out), octets);
   } else {
     return false;
@@ -1119,7 +1130,7 @@ bool launch_dense_16bit(const EltwiseParams& p, int dtype, cudaStream_t stream) 
   d.op = p.op;
   d.n_in = p.n_in;
   d.dtype = dtype;
-  eltwise_16bit_dense_kernel<S><<<grid_for(d.octets), 256, 0, stream>>>(d);
+  launch_dependent(eltwise_16bit_dense_kernel<S>, grid_for(d.octets), 256, stream, d);
   return true;
 }
 }  // namespace
@@ -1133,7 +1144,7 @@ cudaError_t launch_eltwise(const EltwiseParams& p, cudaStream_t stream) {
   DenseF32 dense{};
   if (dense_f32_form(p, &dense)) {
     const long long threads = (dense.quads + 1) / 2;
-    eltwise_f32_dense_kernel<<<grid_for(threads), 256, 0, stream>>>(dense, threads);
+    launch_dependent(eltwise_f32_dense_kernel, grid_for(threads), 256, stream, dense, threads);
     return cudaGetLastError();
   }
   // every operand dense like the result or a single value?
@@ -1160,10 +1171,10 @@ cudaError_t launch_eltwise(const EltwiseParams& p, cudaStream_t stream) {
       const long long threads = (p.elems + 3) / 4;
       const unsigned g4 = grid_for(threads);
       switch (p.compute_class) {
-        case kClassF32: eltwise_dense_kernel<float><<<g4, 256, 0, stream>>>(p, one_value, threads); break;
-        case kClassF64: eltwise_dense_kernel<double><<<g4, 256, 0, stream>>>(p, one_value, threads); break;
-        case kClassI64: eltwise_dense_kernel<long long><<<g4, 256, 0, stream>>>(p, one_value, threads); break;
-        case kClassU64: eltwise_dense_kernel<unsigned long long><<<g4, 256, 0, stream>>>(p, one_value, threads); break;
+        case kClassF32: launch_dependent(eltwise_dense_kernel<float>, g4, 256, stream, p, one_value, threads); break;
+        case kClassF64: launch_dependent(eltwise_dense_kernel<double>, g4, 256, stream, p, one_value, threads); break;
+        case kClassI64: launch_dependent(eltwise_dense_kernel<long long>, g4, 256, stream, p, one_value, threads); break;
+        case kClassU64: launch_dependent(eltwise_dense_kernel<unsigned long long>, g4, 256, stream, p, one_value, threads); break;
         default: return cudaErrorInvalidValue;
       }
       return cudaGetLastError();
@@ -1171,10 +1182,10 @@ cudaError_t launch_eltwise(const EltwiseParams& p, cudaStream_t stream) {
   }
   const unsigned grid = grid_for(p.elems);
   switch (p.compute_class) {
-    case kClassF32: eltwise_kernel<float><<<grid, 256, 0, stream>>>(p); break;
-    case kClassF64: eltwise_kernel<double><<<grid, 256, 0, stream>>>(p); break;
-    case kClassI64: eltwise_kernel<long long><<<grid, 256, 0, stream>>>(p); break;
-    case kClassU64: eltwise_kernel<unsigned long long><<<grid, 256, 0, stream>>>(p); break;
+    case kClassF32: launch_dependent(eltwise_kernel<float>, grid, 256, stream, p); break;
+    case kClassF64: launch_dependent(eltwise_kernel<double>, grid, 256, stream, p); break;
+    case kClassI64: launch_dependent(eltwise_kernel<long long>, grid, 256, stream, p); break;
+    case kClassU64: launch_dependent(eltwise_kernel<unsigned long long>, grid, 256, stream, p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -1182,7 +1193,7 @@ cudaError_t launch_eltwise(const EltwiseParams& p, cudaStream_t stream) {
 
 cudaError_t launch_fill_f32(float* out, long long n, float value, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  fill_kernel<float><<<grid_for(n), 256, 0, stream>>>(out, PMLB_F32, n, value);
+  launch_dependent(fill_kernel<float>, grid_for(n), 256, stream, out, PMLB_F32, n, value);
   return cudaGetLastError();
 }
 

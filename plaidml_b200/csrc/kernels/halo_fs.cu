@@ -1,6 +1,7 @@
 // Compiles and launches the filter-column-merged halo convolution kernel.
 #include "halo_fs_kernel.cuh"
 
+#include "dependent_launch.h"
 #include "halo_fs.h"
 
 namespace pmlb {
@@ -14,8 +15,7 @@ int halo_fs_stages(int weight_bytes, int stage_bytes) {
 
 int halo_fs_tail_bytes() { return kFsTailBytes; }
 
-cudaError_t launch_halo_fs(const TcMaps& maps, const TcParams& p, int grid, int out_bytes, bool pair, bool dependent_launch,
-                           cudaStream_t stream) {
+cudaError_t launch_halo_fs(const TcMaps& maps, const TcParams& p, int grid, int out_bytes, bool pair, cudaStream_t stream) {
   const int wts = p.conv_r * (pair ? 12288 : 24576);
   const int smem = 1024 + wts + p.halo_stages * p.halo_stage_bytes + kFsTailBytes;
   cudaLaunchConfig_t cfg = {};
@@ -32,11 +32,7 @@ cudaError_t launch_halo_fs(const TcMaps& maps, const TcParams& p, int grid, int 
     attr[na].val.clusterDim.z = 1;
     ++na;
   }
-  if (dependent_launch) {
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
+  attr[na++] = dependent_launch_attribute();
   cfg.attrs = attr;
   cfg.numAttrs = na;
   auto go = [&](auto kernel) {

@@ -66,7 +66,6 @@ template <int OB, int CTAS>
 __global__ void __launch_bounds__(kFsThreads, 1)
 conv_halo_fs_kernel(const __grid_constant__ TcMaps tm, const __grid_constant__ TcParams p) {
   const uint32_t cta_rank = CTAS == 2 ? cluster_ctarank() : 0u;
-  grid_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t ring = (raw_addr + 1023u) & ~1023u;
@@ -136,6 +135,7 @@ conv_halo_fs_kernel(const __grid_constant__ TcMaps tm, const __grid_constant__ T
   const uint32_t tmem_base = *tmem_slot;
   // set-up done: from here on the kernel reads and writes tensors, so the kernel before it must be complete
   grid_dependency_wait();
+  grid_launch_dependents();
   if (warp >= 2 && warp < 4) {
     const int ch = (warp - 2) * 32 + lane;
     bias_s[ch] = (p.epi_flags & kEpiBias) ? __ldg(static_cast<const float*>(p.bias) + ch) : 0.f;

@@ -2,6 +2,7 @@
 // multiply (row max, pooling windows, global-average sums).  All of them move 16 bytes
 // per load where alignment allows, keep several loads in flight per thread and finish
 // with warp shuffles; none of them touches the tensor cores.
+#include "dependent_launch.h"
 #include "reduce.h"
 
 #include <type_traits>
@@ -61,6 +62,7 @@ template <class T, class TO, int AGG, bool VEC>
 __global__ void __launch_bounds__(256)
 row_reduce_kernel(const T* __restrict__ in, TO* __restrict__ out, long long rows, long long len,
                   float scale) {
+  dependent_entry();
   using A = typename AccOf<T>::type;
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -114,6 +116,7 @@ template <class T, class TO, int AGG, bool VEC>
 __global__ void __launch_bounds__(256)
 strided_reduce_kernel(const T* __restrict__ in, TO* __restrict__ out, long long outer, long long red,
                       long long inner, float scale) {
+  dependent_entry();
   using A = typename AccOf<T>::type;
   constexpr int N = VEC ? Vec16<T>::N : 1;
   const long long per_outer = inner / N;
@@ -148,6 +151,7 @@ strided_reduce_kernel(const T* __restrict__ in, TO* __restrict__ out, long long 
 template <class T, int AGG, bool VEC>
 __global__ void __launch_bounds__(256)
 pool_kernel(const T* __restrict__ in, T* __restrict__ out, PoolGeom g) {
+  dependent_entry();
   using A = typename AccOf<T>::type;
   constexpr int N = VEC ? Vec16<T>::N : 1;
   const int cv = g.c / N;
@@ -224,6 +228,7 @@ template <class T2, int AGG, bool K3X3, int W>
 __global__ void __launch_bounds__(256)
 pool16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, PoolGeom g, FastDiv fd_cv,
               FastDiv fd_p, uint32_t identity2) {
+  dependent_entry();
   const int cv = g.c / (8 * W);                         // channel groups of one thread's width
   const int pos = blockIdx.y * 256 + threadIdx.x;       // (x, channel group) inside the output row
   if (pos >= g.q * cv) return;
@@ -284,11 +289,11 @@ cudaError_t launch_pool16_w(const PoolGeom& g, const void* in, void* out, uint32
   uint4* op = static_cast<uint4*>(out);
   const bool k3 = g.r == 3 && g.s == 3;
   if (g.agg == PMLB_AGG_MAX) {
-    if (k3) pool16_kernel<T2, PMLB_AGG_MAX, true, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, neg_inf2);
-    else pool16_kernel<T2, PMLB_AGG_MAX, false, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, neg_inf2);
+    if (k3) launch_dependent(pool16_kernel<T2, PMLB_AGG_MAX, true, W>, grid, 256, stream, ip, op, g, fc, fp, neg_inf2);
+    else launch_dependent(pool16_kernel<T2, PMLB_AGG_MAX, false, W>, grid, 256, stream, ip, op, g, fc, fp, neg_inf2);
   } else {
-    if (k3) pool16_kernel<T2, PMLB_AGG_MIN, true, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, pos_inf2);
-    else pool16_kernel<T2, PMLB_AGG_MIN, false, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, pos_inf2);
+    if (k3) launch_dependent(pool16_kernel<T2, PMLB_AGG_MIN, true, W>, grid, 256, stream, ip, op, g, fc, fp, pos_inf2);
+    else launch_dependent(pool16_kernel<T2, PMLB_AGG_MIN, false, W>, grid, 256, stream, ip, op, g, fc, fp, pos_inf2);
   }
   return cudaGetLastError();
 }
@@ -310,18 +315,18 @@ cudaError_t launch_reduce_t(int agg, const void* in, void* out, long long outer,
   if (inner == 1) {
     const unsigned grid = static_cast<unsigned>((outer + 7) / 8);
     switch (agg) {
-      case PMLB_AGG_MAX: row_reduce_kernel<T, TO, PMLB_AGG_MAX, VEC><<<grid, 256, 0, stream>>>(ip, op, outer, red, scale); break;
-      case PMLB_AGG_MIN: row_reduce_kernel<T, TO, PMLB_AGG_MIN, VEC><<<grid, 256, 0, stream>>>(ip, op, outer, red, scale); break;
-      default: row_reduce_kernel<T, TO, PMLB_AGG_SUM, VEC><<<grid, 256, 0, stream>>>(ip, op, outer, red, scale); break;
+      case PMLB_AGG_MAX: launch_dependent(row_reduce_kernel<T, TO, PMLB_AGG_MAX, VEC>, grid, 256, stream, ip, op, outer, red, scale); break;
+      case PMLB_AGG_MIN: launch_dependent(row_reduce_kernel<T, TO, PMLB_AGG_MIN, VEC>, grid, 256, stream, ip, op, outer, red, scale); break;
+      default: launch_dependent(row_reduce_kernel<T, TO, PMLB_AGG_SUM, VEC>, grid, 256, stream, ip, op, outer, red, scale); break;
     }
   } else {
     constexpr int N = VEC ? Vec16<T>::N : 1;
     const long long threads = outer * (inner / N);
     const unsigned grid = static_cast<unsigned>((threads + 255) / 256);
     switch (agg) {
-      case PMLB_AGG_MAX: strided_reduce_kernel<T, TO, PMLB_AGG_MAX, VEC><<<grid, 256, 0, stream>>>(ip, op, outer, red, inner, scale); break;
-      case PMLB_AGG_MIN: strided_reduce_kernel<T, TO, PMLB_AGG_MIN, VEC><<<grid, 256, 0, stream>>>(ip, op, outer, red, inner, scale); break;
-      default: strided_reduce_kernel<T, TO, PMLB_AGG_SUM, VEC><<<grid, 256, 0, stream>>>(ip, op, outer, red, inner, scale); break;
+      case PMLB_AGG_MAX: launch_dependent(strided_reduce_kernel<T, TO, PMLB_AGG_MAX, VEC>, grid, 256, stream, ip, op, outer, red, inner, scale); break;
+      case PMLB_AGG_MIN: launch_dependent(strided_reduce_kernel<T, TO, PMLB_AGG_MIN, VEC>, grid, 256, stream, ip, op, outer, red, inner, scale); break;
+      default: launch_dependent(strided_reduce_kernel<T, TO, PMLB_AGG_SUM, VEC>, grid, 256, stream, ip, op, outer, red, inner, scale); break;
     }
   }
   return cudaGetLastError();
@@ -345,9 +350,9 @@ cudaError_t launch_pool_t(const PoolGeom& g, const void* in, void* out, cudaStre
   const T* ip = static_cast<const T*>(in);
   T* op = static_cast<T*>(out);
   switch (g.agg) {
-    case PMLB_AGG_MAX: pool_kernel<T, PMLB_AGG_MAX, VEC><<<grid, 256, 0, stream>>>(ip, op, g); break;
-    case PMLB_AGG_MIN: pool_kernel<T, PMLB_AGG_MIN, VEC><<<grid, 256, 0, stream>>>(ip, op, g); break;
-    default: pool_kernel<T, PMLB_AGG_SUM, VEC><<<grid, 256, 0, stream>>>(ip, op, g); break;
+    case PMLB_AGG_MAX: launch_dependent(pool_kernel<T, PMLB_AGG_MAX, VEC>, grid, 256, stream, ip, op, g); break;
+    case PMLB_AGG_MIN: launch_dependent(pool_kernel<T, PMLB_AGG_MIN, VEC>, grid, 256, stream, ip, op, g); break;
+    default: launch_dependent(pool_kernel<T, PMLB_AGG_SUM, VEC>, grid, 256, stream, ip, op, g); break;
   }
   return cudaGetLastError();
 }

@@ -77,7 +77,6 @@ __device__ __forceinline__ uint4 sp_max2x4(const uint4& a, const uint4& b) {
 template <bool BF16>
 __global__ void __launch_bounds__(kSpThreads, 1)
 conv_s2d_pool_kernel(const __grid_constant__ S2dPoolParams p) {
-  grid_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t ring = (raw_addr + 1023u) & ~1023u;
@@ -133,6 +132,7 @@ conv_s2d_pool_kernel(const __grid_constant__ S2dPoolParams p) {
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   grid_dependency_wait();
+  grid_launch_dependents();
   if (warp >= 2 && warp < 4) {
     const int ch = (warp - 2) * 32 + lane;
     bias_s[ch] = p.bias != nullptr ? __ldg(p.bias + ch) : 0.f;

@@ -438,7 +438,7 @@ int tc_launch(const TcLaunch& L, cudaStream_t stream, std::string* err) {
       p.fd_wp = make_fastdiv(static_cast<uint32_t>(std::max(1, p.halo_wp)));
       int fs_grid = std::min(p.batch, L.grid_override > 0 ? L.grid_override : num_sms);
       if (fs_pair) fs_grid = 2 * std::max(1, std::min((p.batch + 1) / 2, (L.grid_override > 0 ? L.grid_override : num_sms) / 2));
-      const cudaError_t fe = launch_halo_fs(maps, p, fs_grid, ob_out, fs_pair, dependent_launch_enabled(), stream);
+      const cudaError_t fe = launch_halo_fs(maps, p, fs_grid, ob_out, fs_pair, stream);
       if (fe != cudaSuccess) {
         *err = std::string("kernel launch failed: ") + cudaGetErrorString(fe);
         return 2;

@@ -25,6 +25,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "dependent_launch.h"
 #include "ptx.cuh"
 #include "tc_gemm.cuh"
 
@@ -411,18 +412,6 @@ __device__ __forceinline__ float epi_apply(const TcParams& p, uint32_t (&v)[CW],
   return chunk_best;
 }
 
-// PMLB_TC_DEPENDENT_LAUNCH=1 in the environment launches the tensor-core kernels with the programmatic
-// stream-serialization attribute (see grid_dependency_wait).  Off by default: measured on ResNet-50 it moved
-// a pass by -2 % to +1 %, i.e. within the run-to-run spread (one CTA per SM at 227 KB of shared memory leaves
-// nothing for the next kernel's CTAs to overlap with until an SM is vacated).
-inline bool dependent_launch_enabled() {
-  static const bool on = [] {
-    const char* v = std::getenv("PMLB_TC_DEPENDENT_LAUNCH");
-    return v && v[0] == '1';
-  }();
-  return on;
-}
-
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 tc_contract_kernel(const __grid_constant__ TcMaps tm, const __grid_constant__ TcParams p) {
@@ -432,9 +421,6 @@ tc_contract_kernel(const __grid_constant__ TcMaps tm, const __grid_constant__ Tc
   constexpr int NSPLIT = Cfg::NSPLIT;
   constexpr bool IS_INT = (Cfg::KIND == kMmaI8);
 
-  // (the next kernel of the stream may be scheduled onto SMs as this one leaves them; it waits for this
-  // kernel's completion before it touches memory)
-  grid_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t ring = (raw_addr + 1023u) & ~1023u;           // shared-space address
@@ -525,6 +511,7 @@ tc_contract_kernel(const __grid_constant__ TcMaps tm, const __grid_constant__ Tc
   const uint32_t tmem_base = *tmem_slot;
   // set-up done: from here on the kernel reads and writes tensors, so the kernel before it must be complete
   grid_dependency_wait();
+  grid_launch_dependents();   // (the next kernel's set-up on SMs as this one leaves them)
 
   // (pairs: p.tiles_m counts 256-row pair tiles; CTA `rank` takes rows 128 * rank .. of each)
   const int total_tiles = 2 * p.batch * p.tiles_m * p.tiles_n - p.tiles_full;   // halves count twice
@@ -1585,12 +1572,7 @@ cudaError_t launch_cfg(const TcMaps& maps, const TcParams& p, int grid, cudaStre
     attr[na].val.clusterDim.z = 1;
     ++na;
   }
-  if (dependent_launch_enabled()) {
-    // the kernel's set-up may overlap the tail of the kernel before it (see grid_dependency_wait)
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
+  attr[na++] = dependent_launch_attribute();
   cfg.attrs = attr;
   cfg.numAttrs = na;
   return cudaLaunchKernelEx(&cfg, tc_contract_kernel<Cfg>, maps, p);

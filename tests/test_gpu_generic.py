@@ -559,3 +559,49 @@ def test_product_that_does_not_cover_its_output_or_reads_out_of_range_stays_exac
         d.src[1] = K.make_access(K.F32, [64, 60], [{2: 1}, {1: 1}])
         out, ref = run_contract(d, [a, b], (rows, 60), K.F32)
         np.testing.assert_array_equal(out, ref)
+
+
+@pytest.mark.parametrize("graph", [False, True], ids=["stream", "graph"])
+def test_a_chain_of_short_launches_reads_what_the_launch_before_wrote(graph):
+    # launches may begin before their predecessor has ended: two buffers written in turn by element-wise steps and by
+    # products with a permutation (exact), 200 launches
+    rows, n = 256, 128
+    perm = torch.eye(n, device="cuda")[torch.arange(n).roll(1)].contiguous()
+    one = torch.ones(1, device="cuda")
+    x0 = torch.randint(0, 1000, (rows, n), device="cuda").float()
+
+    e = K.EltwiseDesc()
+    e.op, e.n_in, e.rank, e.out_dtype = b"add", 2, 2, K.F32
+    e.in_dtype[0] = e.in_dtype[1] = K.F32
+    e.sizes[0], e.sizes[1] = rows, n
+    e.in_strides[0][0], e.in_strides[0][1] = n, 1
+    add = K.Plan("eltwise", e)
+    d = K.GemmDesc()
+    d.in_dtype = d.out_dtype = K.F32
+    d.m, d.n, d.k, d.batch = rows, n, n, 1
+    d.lda, d.ldb, d.ldc = n, n, n
+    mul = K.Plan("gemm", d)
+
+    x, y = x0.clone(), torch.empty_like(x0)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+
+    def chain():
+        for _ in range(50):
+            add.eltwise([ptr(x), ptr(one)], ptr(y), stream=stream.cuda_stream)
+            mul.gemm(ptr(y), ptr(perm), ptr(x), stream=stream.cuda_stream)
+            add.eltwise([ptr(x), ptr(one)], ptr(y), stream=stream.cuda_stream)
+            add.eltwise([ptr(y), ptr(one)], ptr(x), stream=stream.cuda_stream)
+
+    with torch.cuda.stream(stream):
+        if graph:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                chain()
+            g.replay()
+        else:
+            chain()
+    stream.synchronize()
+    got = x.cpu()
+    moved = x0.cpu().numpy() @ np.linalg.matrix_power(perm.cpu().numpy(), 50) + 150
+    np.testing.assert_array_equal(got.numpy(), moved.astype(np.float32))
