@@ -6,6 +6,10 @@
 // themselves only after their own wait: at most two neighbours are ever in flight, and a kernel cannot have begun on an
 // SM whose read-only cache the kernel before the last one is still filling.
 //
+// Not for kernels that live on L1 hits (pooling, contractions without tensor cores, operand splitting): beside a
+// tensor-core kernel an SM keeps the carve-out for its shared memory, and they would run with what little L1 is left, as
+// predecessor or as successor (a 4000 x 4000 x 130 product with its operand splitting 58 -> 74 us).
+//
 // Measured on replayed ResNet-50 passes (57 launches of 4 to 17 us at 16 images): batch 1 399 -> 363 us, 4 455 -> 408,
 // 16 559 -> 514, 64 1016 -> 984, 256 2743 -> 2738; an int8 GEMM of 64 x 64 x 128 4.2 -> 3.5 us, 4096^3 50.2 -> 49.5 us.
 // It pays where launches are short and costs nothing where they are long.

@@ -71,7 +71,6 @@ __device__ __forceinline__ long long floor_div_exact(long long num, int den, boo
 
 template <class T>
 __global__ void __launch_bounds__(256) contract_kernel(const __grid_constant__ GenericParams p) {
-  dependent_entry();
   const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= p.out_elems) return;
 
@@ -305,7 +304,6 @@ __device__ __forceinline__ void lean_clip(int c, int step, int size, int* lo, in
 // 86 us, and 6 us on one image (142 us before).
 template <int V>
 __global__ void __launch_bounds__(256) contract_lean_f32_kernel(const __grid_constant__ LeanParams p) {
-  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (t * V >= p.elems) return;
   const LeanPlace w = lean_place(p, static_cast<int>(t * V));
@@ -434,7 +432,6 @@ __device__ __forceinline__ RunVec<W> run_load(const float* p) {
 template <int W, bool ONE_M, bool ONE_F, int NT>
 __global__ void __launch_bounds__(kRunBlock, 1024 / kRunBlock)
 contract_lean_run_kernel(const __grid_constant__ LeanParams p, const __grid_constant__ LeanRun r) {
-  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * kRunBlock + threadIdx.x;
   if (t >= r.threads) return;
   const int last = p.rank - 1, along = p.rank - 2;
@@ -563,7 +560,6 @@ contract_lean_run_kernel(const __grid_constant__ LeanParams p, const __grid_cons
 // The same for any element types, one element per thread, values in the class of the output type.
 template <class T>
 __global__ void __launch_bounds__(256) contract_lean_kernel(const __grid_constant__ LeanParams p) {
-  dependent_entry();
   const long long t = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (t >= p.elems) return;
   const LeanPlace w = lean_place(p, static_cast<int>(t));
@@ -905,10 +901,10 @@ cudaError_t launch_contract(const GenericParams& p, cudaStream_t stream) {
   if (p.out_elems <= 0) return cudaSuccess;
   const unsigned grid = grid_for(p.out_elems);
   switch (dtype_class(p.out.dtype)) {
-    case kClassF32: launch_dependent(contract_kernel<float>, grid, 256, stream, p); break;
-    case kClassF64: launch_dependent(contract_kernel<double>, grid, 256, stream, p); break;
-    case kClassI64: launch_dependent(contract_kernel<long long>, grid, 256, stream, p); break;
-    case kClassU64: launch_dependent(contract_kernel<unsigned long long>, grid, 256, stream, p); break;
+    case kClassF32: contract_kernel<float><<<grid, 256, 0, stream>>>(p); break;
+    case kClassF64: contract_kernel<double><<<grid, 256, 0, stream>>>(p); break;
+    case kClassI64: contract_kernel<long long><<<grid, 256, 0, stream>>>(p); break;
+    case kClassU64: contract_kernel<unsigned long long><<<grid, 256, 0, stream>>>(p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -948,9 +944,9 @@ template <int W, bool ONE_M, bool ONE_F>
 void launch_run(const LeanParams& p, const LeanRun& r, cudaStream_t stream) {
   const unsigned grid = static_cast<unsigned>((r.threads + kRunBlock - 1) / kRunBlock);
   if (r.n_clip <= 1 && r.n_test <= 1) {
-    launch_dependent(contract_lean_run_kernel<W, ONE_M, ONE_F, 1>, grid, kRunBlock, stream, p, r);
+    contract_lean_run_kernel<W, ONE_M, ONE_F, 1><<<grid, kRunBlock, 0, stream>>>(p, r);
   } else {
-    launch_dependent(contract_lean_run_kernel<W, ONE_M, ONE_F, 4>, grid, kRunBlock, stream, p, r);
+    contract_lean_run_kernel<W, ONE_M, ONE_F, 4><<<grid, kRunBlock, 0, stream>>>(p, r);
   }
 }
 }  // namespace
@@ -980,18 +976,18 @@ cudaError_t launch_contract_lean(const LeanParams& p, cudaStream_t stream) {
       else if (one_f) launch_run<4, false, true>(p, run, stream);
       else launch_run<4, false, false>(p, run, stream);
     } else if (quads) {
-      launch_dependent(contract_lean_f32_kernel<4>, grid_for(p.elems / 4), 256, stream, p);
+      contract_lean_f32_kernel<4><<<grid_for(p.elems / 4), 256, 0, stream>>>(p);
     } else {
-      launch_dependent(contract_lean_f32_kernel<1>, grid_for(p.elems), 256, stream, p);
+      contract_lean_f32_kernel<1><<<grid_for(p.elems), 256, 0, stream>>>(p);
     }
     return cudaGetLastError();
   }
   const unsigned grid = grid_for(p.elems);
   switch (dtype_class(p.out_dtype)) {
-    case kClassF32: launch_dependent(contract_lean_kernel<float>, grid, 256, stream, p); break;
-    case kClassF64: launch_dependent(contract_lean_kernel<double>, grid, 256, stream, p); break;
-    case kClassI64: launch_dependent(contract_lean_kernel<long long>, grid, 256, stream, p); break;
-    case kClassU64: launch_dependent(contract_lean_kernel<unsigned long long>, grid, 256, stream, p); break;
+    case kClassF32: contract_lean_kernel<float><<<grid, 256, 0, stream>>>(p); break;
+    case kClassF64: contract_lean_kernel<double><<<grid, 256, 0, stream>>>(p); break;
+    case kClassI64: contract_lean_kernel<long long><<<grid, 256, 0, stream>>>(p); break;
+    case kClassU64: contract_lean_kernel<unsigned long long><<<grid, 256, 0, stream>>>(p); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();

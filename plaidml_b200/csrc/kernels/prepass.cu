@@ -29,7 +29,6 @@ __global__ void __launch_bounds__(256)
 split_tf32_kernel(const float* __restrict__ in, long long ld, long long in_batch,
                   float* __restrict__ hi, float* __restrict__ lo, long long out_ld,
                   long long out_batch, int rows, int cols, bool transpose) {
-  dependent_entry();
   __shared__ float tile[32][33];
   split_tf32_tile(tile, blockIdx.z, blockIdx.x, blockIdx.y, in, ld, in_batch, hi, lo, out_ld, out_batch, rows,
                   cols, transpose);
@@ -39,7 +38,6 @@ split_tf32_kernel(const float* __restrict__ in, long long ld, long long in_batch
 // (padded) extent return at once.
 __global__ void __launch_bounds__(256)
 split_tf32_pair_kernel(SplitTf32Args a, SplitTf32Args b, int a_gx, int a_gy, int b_gx, int b_gy) {
-  dependent_entry();
   __shared__ float tile[32][33];
   const bool first = static_cast<int>(blockIdx.z) < a.batch;
   const SplitTf32Args& s = first ? a : b;
@@ -64,7 +62,6 @@ __device__ __forceinline__ void split4(const float4& v, float4* h, float4* l) {
 // transposed one is read in rows of the input and written in rows of the output.
 __global__ void __launch_bounds__(256)
 split_tf32_pair64_kernel(SplitTf32Args a, SplitTf32Args b, int a_gx, int a_gy, int b_gx, int b_gy) {
-  dependent_entry();
   __shared__ float tile[64][65];
   const bool first = static_cast<int>(blockIdx.z) < a.batch;
   const SplitTf32Args& s = first ? a : b;
@@ -216,7 +213,6 @@ filter_relayout_split_kernel(const void* __restrict__ in, int in_dtype, float* _
 __global__ void __launch_bounds__(256)
 pack_rows_kernel(const uint16_t* __restrict__ in, uint4* __restrict__ out, long long rows, int w,
                  int c, int wp, int cp8, int pad_w) {
-  dependent_entry();
   const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long total = rows * wp * cp8;
   if (id >= total) return;
@@ -411,8 +407,7 @@ cudaError_t launch_pack_rows(const void* in, void* out, int n, int h, int w, int
   const long long rows = static_cast<long long>(n) * h;
   const long long total = rows * wp * (cp / 8);
   if (total <= 0) return cudaSuccess;
-  launch_dependent(pack_rows_kernel, static_cast<unsigned>((total + 255) / 256), 256, stream,
-      static_cast<const uint16_t*>(in), static_cast<uint4*>(out), rows, w, c, wp, cp / 8, pad_w);
+  pack_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(      static_cast<const uint16_t*>(in), static_cast<uint4*>(out), rows, w, c, wp, cp / 8, pad_w);
   return cudaGetLastError();
 }
 
@@ -434,7 +429,7 @@ cudaError_t launch_split_tf32(const float* in, long long ld, long long in_batch,
   const int cover_rows = transpose ? out_cols : out_rows;  // in input-row units
   const int cover_cols = transpose ? out_rows : out_cols;  // in input-col units
   dim3 grid((cover_cols + 31) / 32, (cover_rows + 31) / 32, batch);
-  launch_dependent(split_tf32_kernel, grid, 256, stream, in, ld, in_batch, hi, lo, out_ld, out_batch, rows,
+  split_tf32_kernel<<<grid, 256, 0, stream>>>(in, ld, in_batch, hi, lo, out_ld, out_batch, rows,
                                               cols, transpose);
   return cudaGetLastError();
 }
@@ -466,7 +461,7 @@ cudaError_t launch_split_tf32_pair(const SplitTf32Args& a, const SplitTf32Args& 
     const int ax = (agx + 1) / 2, ay = (agy + 1) / 2, bx = (bgx + 1) / 2, by = (bgy + 1) / 2;   // 64-wide tiles
     dim3 grid64(ax > bx ? ax : bx, ay > by ? ay : by, a.batch + b.batch);
     if (grid64.y <= 65535u && grid64.z <= 65535u) {
-      launch_dependent(split_tf32_pair64_kernel, grid64, 256, stream, a, b, ax, ay, bx, by);
+      split_tf32_pair64_kernel<<<grid64, 256, 0, stream>>>(a, b, ax, ay, bx, by);
       return cudaGetLastError();
     }
   }
@@ -478,7 +473,7 @@ cudaError_t launch_split_tf32_pair(const SplitTf32Args& a, const SplitTf32Args& 
     return launch_split_tf32(b.in, b.ld, b.in_batch, b.hi, b.lo, b.out_ld, b.out_batch, b.rows, b.cols, b.batch,
                              b.transpose, stream);
   }
-  launch_dependent(split_tf32_pair_kernel, grid, 256, stream, a, b, agx, agy, bgx, bgy);
+  split_tf32_pair_kernel<<<grid, 256, 0, stream>>>(a, b, agx, agy, bgx, bgy);
   return cudaGetLastError();
 }
 

@@ -151,7 +151,6 @@ strided_reduce_kernel(const T* __restrict__ in, TO* __restrict__ out, long long 
 template <class T, int AGG, bool VEC>
 __global__ void __launch_bounds__(256)
 pool_kernel(const T* __restrict__ in, T* __restrict__ out, PoolGeom g) {
-  dependent_entry();
   using A = typename AccOf<T>::type;
   constexpr int N = VEC ? Vec16<T>::N : 1;
   const int cv = g.c / N;
@@ -228,7 +227,6 @@ template <class T2, int AGG, bool K3X3, int W>
 __global__ void __launch_bounds__(256)
 pool16_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, PoolGeom g, FastDiv fd_cv,
               FastDiv fd_p, uint32_t identity2) {
-  dependent_entry();
   const int cv = g.c / (8 * W);                         // channel groups of one thread's width
   const int pos = blockIdx.y * 256 + threadIdx.x;       // (x, channel group) inside the output row
   if (pos >= g.q * cv) return;
@@ -289,11 +287,11 @@ cudaError_t launch_pool16_w(const PoolGeom& g, const void* in, void* out, uint32
   uint4* op = static_cast<uint4*>(out);
   const bool k3 = g.r == 3 && g.s == 3;
   if (g.agg == PMLB_AGG_MAX) {
-    if (k3) launch_dependent(pool16_kernel<T2, PMLB_AGG_MAX, true, W>, grid, 256, stream, ip, op, g, fc, fp, neg_inf2);
-    else launch_dependent(pool16_kernel<T2, PMLB_AGG_MAX, false, W>, grid, 256, stream, ip, op, g, fc, fp, neg_inf2);
+    if (k3) pool16_kernel<T2, PMLB_AGG_MAX, true, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, neg_inf2);
+    else pool16_kernel<T2, PMLB_AGG_MAX, false, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, neg_inf2);
   } else {
-    if (k3) launch_dependent(pool16_kernel<T2, PMLB_AGG_MIN, true, W>, grid, 256, stream, ip, op, g, fc, fp, pos_inf2);
-    else launch_dependent(pool16_kernel<T2, PMLB_AGG_MIN, false, W>, grid, 256, stream, ip, op, g, fc, fp, pos_inf2);
+    if (k3) pool16_kernel<T2, PMLB_AGG_MIN, true, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, pos_inf2);
+    else pool16_kernel<T2, PMLB_AGG_MIN, false, W><<<grid, 256, 0, stream>>>(ip, op, g, fc, fp, pos_inf2);
   }
   return cudaGetLastError();
 }
@@ -350,9 +348,9 @@ cudaError_t launch_pool_t(const PoolGeom& g, const void* in, void* out, cudaStre
   const T* ip = static_cast<const T*>(in);
   T* op = static_cast<T*>(out);
   switch (g.agg) {
-    case PMLB_AGG_MAX: launch_dependent(pool_kernel<T, PMLB_AGG_MAX, VEC>, grid, 256, stream, ip, op, g); break;
-    case PMLB_AGG_MIN: launch_dependent(pool_kernel<T, PMLB_AGG_MIN, VEC>, grid, 256, stream, ip, op, g); break;
-    default: launch_dependent(pool_kernel<T, PMLB_AGG_SUM, VEC>, grid, 256, stream, ip, op, g); break;
+    case PMLB_AGG_MAX: pool_kernel<T, PMLB_AGG_MAX, VEC><<<grid, 256, 0, stream>>>(ip, op, g); break;
+    case PMLB_AGG_MIN: pool_kernel<T, PMLB_AGG_MIN, VEC><<<grid, 256, 0, stream>>>(ip, op, g); break;
+    default: pool_kernel<T, PMLB_AGG_SUM, VEC><<<grid, 256, 0, stream>>>(ip, op, g); break;
   }
   return cudaGetLastError();
 }
