@@ -5,14 +5,14 @@
 // of 8, and bf16 operands may be MN-major, so a [k][n] B or a transposed A needs no transposition.
 //
 // One CTA computes a 128 x BN tile (or the part of its K range that falls to it, see below):
-//   warps 0..7   loaders: fp32 from global memory into registers one operand tile ahead, cut into the three parts,
+//   warps 0..15  loaders: fp32 from global memory into registers one operand tile ahead, cut into the three parts,
 //                stored in the 128-byte swizzle the MMA reads.  No pre-pass writes and re-reads split copies, and
 //                any row alignment is accepted.
-//   warp 16      MMA issuer.  hh goes into an accumulator of its own; the five small products share a second one:
+//   warp 24      MMA issuer.  hh goes into an accumulator of its own; the five small products share a second one:
 //                the tensor core truncates when it adds to its accumulator, an error per MMA of a fraction of the
 //                accumulator's last place, and the small sums must not drown in it.  [h | m] of B lie side by side
 //                in shared memory, so one MMA of width 2 BN does hh and hm with one read of A.
-//   warps 8..15  after every kFlushBlocks k-blocks (256 terms) they add both accumulators to sums in registers with
+//   warps 16..23 after every kFlushBlocks k-blocks (256 terms) they add both accumulators to sums in registers with
 //                round-to-nearest while the issuer goes on with the other accumulator pair: chains of 16 MMAs instead
 //                of k / 8.  Error against 64 bits at 2048 terms: 2.3e-7, three TF32 products in one chain 1.4e-5.
 //   all warps    the sums go through shared memory (free by then) to row-contiguous 16-byte stores with the epilogue.
@@ -21,14 +21,18 @@
 // adds a 128 / split-row strip of all parts through distributed shared memory, in rank order.  No scratch memory, no
 // atomics, no second launch; the result depends only on the shape.
 //
-// What bounds it: 64- and 128-wide tiles the SM's 128 bytes per cycle of shared memory (per k-block of a 128-wide tile
-// 176 KB of operand reads by the MMAs, 98 KB of stores by the loaders and 64 KB of loads: 2400 cycles where the MMAs
-// alone take 1536); CTA pairs (256 x 256 tiles, each operand element read by half as many MMAs) the rate the tensor
-// pipe sustains under the power limit (six products of 2048 x 2048 x 1024 in 41 us: 1.27 PFLOP/s, 1.6 in the loop).
-// Measured (graph replays), split copies by a pre-pass -> here: 1 x 1000 x 2048 35 -> 12 us, 300^3 12.9 -> 8.0, 1024^3
-// 22.0 -> 19.2, 512 x 512 x 4096 62 -> 24, 1999 x 2001 x 1001 71 -> 55, convolution 8 x 28 x 28 x 128 -> 128, 3x3 25.6
-// -> 22.1, 1 x 7 x 7 x 512 -> 512, 3x3 61 -> 17.  Walking several tiles per CTA with the stores behind the next tile's
-// loads was slower (1024^3 21.2 us): stores, loads and operands share the same bytes per cycle.
+// CTA pairs (256 x 256 tiles) have room for one accumulator pair only: their chains run over the pair's whole part of K.
+//
+// What bounds it: 64- and 128-wide tiles the loaders: per k-block of a 128-wide tile 64 KB of loads, 98 KB of stores and
+// 16,384 elements to cut (18 instructions per four), ~2300 cycles where the MMAs take 1536; leaving out the loads or
+// the stores saves a quarter each, leaving out half of the MMAs 6 %.  Eight loader warps instead of 16 cost 2-8 %;
+// offsets that stay in registers and packed additions took 40 instructions per four elements to 22 and another 3-10 %.
+// CTA pairs: the rate the tensor pipe sustains under the power limit (six products of 2048 x 2048 x 1024 in 41 us:
+// 1.27 PFLOP/s, 1.6 in the loop).  Small problems: ~6 us of launch, first loads, last sums and stores.
+// Measured (graph replays), split copies by a pre-pass -> here: 1 x 1000 x 2048 35 -> 11.5 us, 300^3 12.9 -> 7.1, 1024^3
+// 22.0 -> 18.2, 256 x 4096 x 4096 96 -> 49, 512 x 512 x 4096 62 -> 22, 1999 x 2001 x 1001 71 -> 49; convolutions 8 x 28 x
+// 28 x 128 -> 128, 3x3 25.5 -> 20.0, 32 x 7 x 7 x 512 -> 512, 3x3 63 -> 45 (pairs, K in parts), 1 x 7 x 7 x 512 61 -> 15.
+// Walking several tiles per CTA with the stores behind the next tile's loads was slower (1024^3 21.2 us against 19.2).
 //
 // inf / NaN: x - h is NaN for them, so only hh is right; a sum whose hh part is not finite drops its small part.
 #include "f32_mma.h"
@@ -49,12 +53,12 @@ namespace pmlb {
 
 namespace {
 
-constexpr int kLoaderWarps = 8;
+constexpr int kLoaderWarps = 16;
 constexpr int kSumWarps = 8;
 constexpr int kThreads = (kLoaderWarps + kSumWarps + 4) * 32;   // (whole warpgroups: the issuer's has three idle warps)
-// Registers per thread: 640 threads start with 96 (61,440 in all).  The issuer's warpgroup goes down to 40, which frees
-// 7,168 of them, and the loaders go up to 120, which takes 6,144: both operand tiles in flight without spills.
-constexpr int kIssuerRegs = 40, kLoaderRegs = 120;
+// Registers per thread: 896 threads start with 72 (64,512 in all).  The loaders go down to 64 and the issuer's warpgroup
+// to 40, which frees 8,192; the sums go up to 96, which takes 6,144.
+constexpr int kIssuerRegs = 40, kLoaderRegs = 64, kSumRegs = 96;
 constexpr int kIssuerWarp = kLoaderWarps + kSumWarps;
 constexpr int kBlockK = 64;            // k-block: 64 terms = 128-byte bf16 rows
 constexpr int kFlushBlocks = 4;        // k-blocks per accumulator chain
@@ -121,20 +125,25 @@ __device__ __forceinline__ uint32_t upper_halves(float lo, float hi) {
   return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
 }
 
+// (a, b) + (c, d) in one instruction.
+__device__ __forceinline__ float2 add2(float a, float b, float c, float d) {
+  float2 r;
+  asm("{\n\t"
+      ".reg .b64 x, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t"
+      "}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
+}
+
 // What is left of two floats without their upper halves (exact; NaN for inf).
 __device__ __forceinline__ float2 rest_of(float x, float y) {
-  const float hx = __uint_as_float(__float_as_uint(x) & 0xffff0000u), hy = __uint_as_float(__float_as_uint(y) & 0xffff0000u);
-  float2 d;
-  asm("{\n\t"
-      ".reg .b64 a, b;\n\t"
-      "mov.b64 a, {%2, %3};\n\t"
-      "mov.b64 b, {%4, %5};\n\t"
-      "add.rn.f32x2 a, a, b;\n\t"
-      "mov.b64 {%0, %1}, a;\n\t"
-      "}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(x), "f"(y), "f"(-hx), "f"(-hy));
-  return d;
+  // the upper half with its sign turned: one logic operation
+  return add2(x, y, __uint_as_float((__float_as_uint(x) & 0xffff0000u) ^ 0x80000000u), __uint_as_float((__float_as_uint(y) & 0xffff0000u) ^ 0x80000000u));
 }
 
 __device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t x, uint32_t y) {
@@ -177,6 +186,8 @@ struct TileLoader {
   const float* origin;
   long long ld;
   int rows, k_end;
+  bool plain;                 // whole k-blocks need no tests: see place()
+  uint32_t at[kGroups];       // byte offset of each group from the k-block's first element (rows layouts only)
   // convolution: first tap's position and the image's offset of each of this thread's rows
   int base[LAYOUT == kRowsConv ? kGroups : 1];
   int yx[LAYOUT == kRowsConv ? kGroups : 1];
@@ -214,33 +225,22 @@ struct TileLoader {
     }
   }
 
-  // WHOLE: every group of this tile's existing rows lies inside the operand.
-  template <bool WHOLE>
-  __device__ __forceinline__ void load_as(int k0, const F32MmaParams& p, int tid) {
-    if constexpr (LAYOUT == kRowsK) {
-      const int k = k0 + (tid % kKGroups) * kGroup;
-      const int r0 = tid / kKGroups;
-      const float* q = origin + static_cast<long long>(r0) * ld + k;
-      const int valid_k = k_end - k;
+  // After origin, ld, rows and k_end are set.  A thread's groups keep their places in every k-block, so a load is one
+  // instruction: the block's address is the same for all threads, the offset never changes.  Groups of rows that do not
+  // exist read the first group instead: what they bring reaches only results that are not stored.
+  __device__ __forceinline__ void place(int tid) {
+    plain = rows > 0 && ld < (1 << 23) && (LAYOUT == kRowsK || rows % kGroup == 0);
 #pragma unroll
-      for (int i = 0; i < kGroups; ++i) {
-        const bool row = r0 + kKStep * i < rows;
-        if constexpr (WHOLE) fetch_if(i, q, row);
-        else fetch(i, q, row ? valid_k : 0);
-        q += kKStep * ld;
-      }
-    } else if constexpr (LAYOUT == kRowsMn) {
-      const int mn = (tid % kMnGroups) * kGroup;
-      const int kk = k0 + tid / kMnGroups;
-      const float* q = origin + static_cast<long long>(kk) * ld + mn;
-      const int valid_mn = rows - mn;
-#pragma unroll
-      for (int i = 0; i < kGroups; ++i) {
-        if constexpr (WHOLE) fetch_if(i, q, valid_mn > 0);
-        else fetch(i, q, kk + kMnStep * i < k_end ? valid_mn : 0);
-        q += kMnStep * ld;
-      }
-    } else {
+    for (int i = 0; i < kGroups; ++i) {
+      const int row = LAYOUT == kRowsK ? tid / kKGroups + kKStep * i : (tid % kMnGroups) * kGroup;
+      const int term = LAYOUT == kRowsK ? (tid % kKGroups) * kGroup : tid / kMnGroups + kMnStep * i;
+      const uint32_t r = row < rows ? row : 0;
+      at[i] = 4u * (LAYOUT == kRowsK ? r * static_cast<uint32_t>(ld) + term : term * static_cast<uint32_t>(ld) + r);
+    }
+  }
+
+  __device__ __forceinline__ void load(int k0, const F32MmaParams& p, int tid) {
+    if constexpr (LAYOUT == kRowsConv) {
       const int k = k0 + (tid % kKGroups) * kGroup;
       const int tap = fast_div(k, p.fd_c);
       const int ch = k - tap * p.c;
@@ -254,14 +254,36 @@ struct TileLoader {
         const bool in = live && static_cast<unsigned>(y) < static_cast<unsigned>(p.h) && static_cast<unsigned>(x) < static_cast<unsigned>(p.w);
         fetch_if(i, origin + base[i] + off, in);
       }
-    }
-  }
-
-  __device__ __forceinline__ void load(int k0, const F32MmaParams& p, int tid) {
-    if (LAYOUT == kRowsConv || (k0 + kBlockK <= k_end && (LAYOUT == kRowsK || rows % kGroup == 0))) {
-      load_as<true>(k0, p, tid);
+    } else if (plain && k0 + kBlockK <= k_end) {
+      const char* block = reinterpret_cast<const char*>(origin + (LAYOUT == kRowsK ? k0 : k0 * ld));
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) {
+        if constexpr (VEC) {
+          const float4 u = __ldg(reinterpret_cast<const float4*>(block + at[i]));
+          v[i][0] = u.x, v[i][1] = u.y, v[i][2] = u.z, v[i][3] = u.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < kGroup; ++e) v[i][e] = __ldg(reinterpret_cast<const float*>(block + at[i]) + e);
+        }
+      }
+    } else if constexpr (LAYOUT == kRowsK) {
+      const int k = k0 + (tid % kKGroups) * kGroup;
+      const int r0 = tid / kKGroups;
+      const float* q = origin + static_cast<long long>(r0) * ld + k;
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) {
+        fetch(i, q, r0 + kKStep * i < rows ? k_end - k : 0);
+        q += kKStep * ld;
+      }
     } else {
-      load_as<false>(k0, p, tid);
+      const int mn = (tid % kMnGroups) * kGroup;
+      const int kk = k0 + tid / kMnGroups;
+      const float* q = origin + static_cast<long long>(kk) * ld + mn;
+#pragma unroll
+      for (int i = 0; i < kGroups; ++i) {
+        fetch(i, q, kk + kMnStep * i < k_end ? rows - mn : 0);
+        q += kMnStep * ld;
+      }
     }
   }
 
@@ -333,10 +355,22 @@ __device__ __forceinline__ void setup_done() {
   }
 }
 
-// An accumulator's hh sum with its small products; those of inf / NaN operands are NaN and dropped.
-__device__ __forceinline__ float both_parts(uint32_t hh, uint32_t small) {
-  const float main = __uint_as_float(hh);
-  return fabsf(main) < INFINITY ? main + __uint_as_float(small) : main;
+// Accumulators' hh sums with their small products; those of inf / NaN operands are NaN and dropped.
+template <int N>
+__device__ __forceinline__ void both_parts(const uint32_t (&hh)[N], const uint32_t (&small)[N], float (&v)[N]) {
+  bool nan = false;
+#pragma unroll
+  for (int e = 0; e < N; e += 2) {
+    const float2 t = add2(__uint_as_float(hh[e]), __uint_as_float(hh[e + 1]), __uint_as_float(small[e]), __uint_as_float(small[e + 1]));
+    v[e] = t.x, v[e + 1] = t.y;
+    nan = nan || t.x != t.x || t.y != t.y;
+  }
+  if (nan) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      if (!(fabsf(__uint_as_float(hh[e])) < INFINITY)) v[e] = __uint_as_float(hh[e]);
+    }
+  }
 }
 
 // Bias, residual, ReLU and the store of `n` <= 4 consecutive results of row i from column j on.
@@ -408,28 +442,32 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
     fence_mbar_init();
   }
   // this CTA's tile and its run of k-blocks
-  const int share = PAIR ? 2 : p.split;          // CTAs per tile
+  // (the CTAs of a tile are one cluster: `split` parts of K, of a pair each where the tile is a pair's)
+  const int share = PAIR ? 2 * p.split : p.split;
   const int unit = static_cast<int>(blockIdx.x) / share;
-  const int rank = static_cast<int>(blockIdx.x) - unit * share;
+  const int cluster_rank = static_cast<int>(blockIdx.x) - unit * share;
+  const int rank = PAIR ? cluster_rank >> 1 : cluster_rank;   // part of K
+  const int side = PAIR ? cluster_rank & 1 : 0;               // CTA of the pair
+  const uint32_t first_cta = static_cast<uint32_t>(cluster_rank & ~1);
   const int batch = unit / p.tiles_per_batch;
   const int tile = unit - batch * p.tiles_per_batch;
   const int tm = tile / p.tiles_n;
-  const int m0 = PAIR ? tm * 256 + rank * 128 : tm * 128;
+  const int m0 = PAIR ? tm * 256 + side * 128 : tm * 128;
   const int n0 = (tile - tm * p.tiles_n) * BN;
-  const int kb_begin = PAIR ? 0 : static_cast<int>(static_cast<long long>(p.num_kb) * rank / p.split);
-  const int kb_end = PAIR ? p.num_kb : static_cast<int>(static_cast<long long>(p.num_kb) * (rank + 1) / p.split);
+  const int kb_begin = static_cast<int>(static_cast<long long>(p.num_kb) * rank / p.split);
+  const int kb_end = static_cast<int>(static_cast<long long>(p.num_kb) * (rank + 1) / p.split);
   const int blocks = kb_end - kb_begin;
 
   if (warp < kLoaderWarps) {
     // ------------------------------------------------------------ loaders
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kLoaderRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLoaderRegs));
     const int tid = threadIdx.x;
     TileLoader<AL, 128, VEC> la;
     TileLoader<BL, BR, VEC> lb;
     la.k_end = lb.k_end = p.k;
     la.ld = p.lda;
     lb.ld = p.ldb;
-    const int nb0 = PAIR ? n0 + rank * BR : n0;    // first column of B this CTA loads
+    const int nb0 = PAIR ? n0 + side * BR : n0;    // first column of B this CTA loads
     la.rows = min(128, p.m - m0);
     lb.rows = min(BR, p.n - nb0);
     if constexpr (AL == kRowsConv) {
@@ -453,6 +491,8 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
       la.origin = p.a + batch * p.a_batch + (AL == kRowsMn ? static_cast<long long>(m0) : static_cast<long long>(m0) * p.lda);
     }
     lb.origin = p.b + batch * p.b_batch + (BL == kRowsMn ? static_cast<long long>(nb0) : static_cast<long long>(nb0) * p.ldb);
+    if constexpr (AL != kRowsConv) la.place(tid);
+    lb.place(tid);
     grid_dependency_wait();
     grid_launch_dependents();
     // (the first loads are on their way while the barriers and TMEM are set up)
@@ -475,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
       __syncwarp();
       if (lane == 0) {
         if constexpr (PAIR) {
-          mbar_arrive_release_cluster(mapa_rank(full_bar(stage), 0));
+          mbar_arrive_release_cluster(mapa_rank(full_bar(stage), first_cta));
         } else {
           mbar_arrive(full_bar(stage));
         }
@@ -510,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
     constexpr uint32_t id2 = mma_desc(PAIR ? BN : 2 * BN, A_MN, B_MN), id3 = mma_desc(3 * 64, A_MN, B_MN);
     int stage = 0;
     uint32_t phase = 0;
-    const bool issues = warp == kIssuerWarp && (!PAIR || rank == 0);
+    const bool issues = warp == kIssuerWarp && (!PAIR || side == 0);
     for (int i = 0; i < blocks && issues; ++i) {
       const bool first = PAIR ? i == 0 : i % kFlushBlocks == 0;
       const bool last = i == blocks - 1 || (!PAIR && i % kFlushBlocks == kFlushBlocks - 1);
@@ -555,8 +595,8 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
           }
         }
         if constexpr (PAIR) {
-          tc_commit_pair(empty_bar(stage), 3);   // the stage is free in both CTAs
-          if (last) tc_commit_pair(tfull_bar(acc), 3);
+          tc_commit_pair(empty_bar(stage), static_cast<uint16_t>(3u << first_cta));   // the stage is free in both CTAs
+          if (last) tc_commit_pair(tfull_bar(acc), static_cast<uint16_t>(3u << first_cta));
         } else {
           tc_commit(empty_bar(stage));
           if (last) tc_commit(tfull_bar(acc));
@@ -569,6 +609,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
     }
   } else {
     // ------------------------------------------------------------ sums
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSumRegs));
     setup_done<2, PAIR>();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
@@ -596,8 +637,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
           tmem_ld_16(t_half + BN + j, small);
           tmem_ld_wait();
           float v[16];
-#pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = both_parts(hh[e], small[e]);
+          both_parts(hh, small, v);
 #pragma unroll
           for (int e = 0; e < 16; e += 4) put(j + e, v[e], v[e + 1], v[e + 2], v[e + 3]);
         }
@@ -627,12 +667,20 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
             tmem_ld_8(t + 2 * BN + j, small2);
             tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 8; ++e) small[e] = __float_as_uint(__uint_as_float(small[e]) + __uint_as_float(small2[e]));
+            for (int e = 0; e < 8; e += 2) {
+              const float2 t = add2(__uint_as_float(small[e]), __uint_as_float(small[e + 1]), __uint_as_float(small2[e]), __uint_as_float(small2[e + 1]));
+              small[e] = __float_as_uint(t.x), small[e + 1] = __float_as_uint(t.y);
+            }
           } else {
             tmem_ld_wait();
           }
+          float v[8];
+          both_parts(hh, small, v);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) sum[j + e] += both_parts(hh[e], small[e]);
+          for (int e = 0; e < 8; e += 2) {
+            const float2 t = add2(sum[j + e], sum[j + e + 1], v[e], v[e + 1]);
+            sum[j + e] = t.x, sum[j + e + 1] = t.y;
+          }
         }
         tc_fence_before_sync();
         __syncwarp();
@@ -648,7 +696,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
   // ---------------------------------------------------------------- parts of the tile -> output
   __syncwarp();
   tc_fence_before_sync();
-  const int strips = PAIR ? 1 : p.split;   // row strips that the tile's CTAs add up and store
+  const int strips = p.split;   // row strips that the CTAs of a tile (of a pair's side) add up and store
   if (strips > 1) {
     cluster_sync_each_thread();
   } else {
@@ -670,7 +718,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
       float o[4] = {0.f, 0.f, 0.f, 0.f};
       if (strips > 1) {
         for (int r = 0; r < strips; ++r) {
-          const float4 u = ld_cluster_v4(mapa_rank(at, static_cast<uint32_t>(r)));
+          const float4 u = ld_cluster_v4(mapa_rank(at, static_cast<uint32_t>(PAIR ? 2 * r + side : r)));
           o[0] += u.x, o[1] += u.y, o[2] += u.z, o[3] += u.w;
         }
       } else {
@@ -770,9 +818,8 @@ struct Choice {
 };
 
 // Tile width and K split: the pair with the smallest estimated time, in cycles per wave of resident tiles.  Measured
-// (B200, 1.9 GHz): a k-block takes 1700 cycles with 64-wide and 2400 with 128-wide tiles (their products' operand
-// reads, the loaders' stores and the loads share the SM's 128 bytes per cycle) and 3750 on a CTA pair for four times
-// the 128-wide tile's work on two SMs (the rate the tensor pipe sustains); rows that are not 16-byte aligned cost a
+// (B200, 1.9 GHz): a k-block takes 1700 cycles with 64-wide and 2400 with 128-wide tiles (the loaders) and 3750 on a CTA
+// pair for four times the 128-wide tile's work on two SMs (the rate the tensor pipe sustains); rows that are not 16-byte aligned cost a
 // third more loads.  Everything around the loop: 8800, 11500 and 18000 cycles, and 1500 + 150 per CTA of a K split.
 Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_override, int split_override, bool pairs, int dev, int sms) {
   Choice best;
@@ -780,13 +827,13 @@ Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_overri
     if (bn_override != 0 && bn != bn_override) continue;
     const int rows = bn == 256 ? 256 : 128;
     const long long tiles = static_cast<long long>((m + rows - 1) / rows) * ((n + bn - 1) / bn) * batch;
-    for (int split = 1; split <= (bn == 256 ? 1 : 8); ++split) {
-      if (bn == 256 ? split_override > 1 : (split_override != 0 ? split != split_override : split > num_kb)) continue;
-      const int share = bn == 256 ? 2 : split;
+    for (int split = 1; split <= (bn == 256 ? 4 : 8); ++split) {
+      if (split_override != 0 ? split != split_override : split > num_kb) continue;
+      const int share = bn == 256 ? 2 * split : split;
       const long long room = share == 1 ? sms : resident_clusters(dev, share);
       const long long waves = (tiles + room - 1) / room;
       const double block = (bn == 256 ? 3750.0 : (bn == 128 ? 2400.0 : 1700.0)) * (vec ? 1.0 : 1.33);
-      const double around = bn == 256 ? 18000.0 : (bn == 128 ? 11500.0 : 8800.0) + (split > 1 ? 1500.0 + 150.0 * split : 0.0);
+      const double around = (bn == 256 ? 18000.0 : (bn == 128 ? 11500.0 : 8800.0)) + (split > 1 ? 1500.0 + 150.0 * split : 0.0);
       const double cycles = static_cast<double>(waves) * ((num_kb + split - 1) / split * block + around);
       if (best.bn == 0 || cycles < best.cycles) {
         best.bn = bn;
@@ -841,7 +888,7 @@ bool f32_mma_faster(const F32MmaShape& s, F32MmaTiles* tiles) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const Choice any = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, true, dev, sms);
-  const double here = any.cycles / 1900.0 * (s.conv ? 1.2 : 1.0);
+  const double here = any.cycles / 1900.0 * (s.conv ? (any.bn == 256 ? 1.05 : 1.2) : 1.0);   // (gathering pixels costs more)
   *tiles = f32_mma_tiles(s);
   const double tiles_m = (s.m + 127) / 128;
   auto prepass = [&](int bn, double block_us) {
@@ -884,7 +931,7 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   const int best_bn = L.tiles.bn;
   p.split = L.tiles.split;
   p.tiles_n = (L.n + best_bn - 1) / best_bn;
-  const int tile_rows = best_bn == 256 ? 256 : 128, share = best_bn == 256 ? 2 : p.split;
+  const int tile_rows = best_bn == 256 ? 256 : 128, share = best_bn == 256 ? 2 * p.split : p.split;
   const long long per_batch = static_cast<long long>((L.m + tile_rows - 1) / tile_rows) * p.tiles_n;
   const long long units = per_batch * L.batch;
   if (units > 0x0fffffffll) {
