@@ -117,7 +117,7 @@ pmlb_status pmlb_plan_arm_timeout_test(pmlb_plan* plan, int wait_limit_ms);
  * and, for int8 / 16-bit inputs, the plain LLVM loops the x86 target emits for
  * non-f32 contractions (pmlc/target/x86/pipeline.cc:185-202).
  *
- * in_dtype / out_dtype:  F32 -> F32 (three TF32 products per term, f32 accumulate)
+ * in_dtype / out_dtype:  F32 -> F32 (six bf16 part products per term, or three TF32 products; f32 accumulate)
  *                        BF16 or F16 -> F32, BF16 or F16 (f32 accumulate)
  *                        I8 -> I32, or I8 (two's-complement wrap of the 32-bit sum)
  * A batch stride of 0 shares one matrix between all batch entries.

@@ -751,8 +751,8 @@ class Planner {
       if (M.extent > INT32_MAX || N.extent > INT32_MAX || K.extent > INT32_MAX || B.extent > INT32_MAX) continue;
       // batch must be outermost in the output
       if (B.any && M.any && B.strideOut < M.strideOut * M.extent) continue;
-      // A tiny fp32 product gains nothing from the tensor cores (the launch dominates) and would lose the
-      // last bits to the three-TF32-product form; the general kernel computes it in plain f32, which is what
+      // A tiny fp32 product gains nothing from the tensor cores (the launch dominates) and would add its terms in
+      // another order; the general kernel computes it in plain f32, term by term, which is what
       // the reference's exact small-matrix expectations (plaidml/edsl/examples/gemm.cc:79-90) were written for.
       if (inDtype == PMLB_F32 && M.extent * N.extent * K.extent * B.extent <= 32768) return false;
       pmlb_gemm_desc d;
@@ -1147,8 +1147,10 @@ class Planner {
            << (pd.gemm.b_is_nk ? " B[n][k]" : " B[k][n]") << pd.fused;
         if (pmlb_plan_split_k(plan) > 1) os << " splitk=" << pmlb_plan_split_k(plan);
         st.detail = os.str();
-        // (+ the TF32 split of both operands, + the row-max fill, + the combining pass of a split K range)
-        st.launches = 1 + (pd.gemm.in_dtype == PMLB_F32 ? 1 : 0) + (pd.rowmax >= 0 ? 1 : 0) + (pmlb_plan_split_k(plan) > 1 ? 1 : 0);
+        // (+ the TF32 split of both operands where the plan holds room for it, + the row-max fill, + the combining pass
+        // of a split K range)
+        const bool split = pd.gemm.in_dtype == PMLB_F32 && pmlb_plan_scratch_bytes(plan) > 256;
+        st.launches = 1 + (split ? 1 : 0) + (pd.rowmax >= 0 ? 1 : 0) + (pmlb_plan_split_k(plan) > 1 ? 1 : 0);
         const void* a = dev(pd.a);
         const void* a2 = pd.a2 >= 0 ? dev(pd.a2) : nullptr;
         const void* b = pd.bDerived ? pd.bDerived : dev(pd.b);
