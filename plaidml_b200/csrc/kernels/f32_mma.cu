@@ -24,9 +24,11 @@
 // CTA pairs (256 x 256 tiles) have room for one accumulator pair only: their chains run over the pair's whole part of K.
 //
 // What bounds it: 64- and 128-wide tiles the loaders: per k-block of a 128-wide tile 64 KB of loads, 98 KB of stores and
-// 16,384 elements to cut (18 instructions per four), ~2300 cycles where the MMAs take 1536; leaving out the loads or
-// the stores saves a quarter each, leaving out half of the MMAs 6 %.  Eight loader warps instead of 16 cost 2-8 %;
-// offsets that stay in registers and packed additions took 40 instructions per four elements to 22 and another 3-10 %.
+// 16,384 elements to cut, ~2300 cycles where the MMAs take 1536.  Copies of an earlier form (eight loader warps, 1024 x
+// 1024 x 4096, 90.6 us) with work left out: without the loads 71.4 us, without the stores 69.3, with two of the five MMAs
+// 85.3.  Over 73 shapes 16 loader warps instead of eight took -12 to +5 % (median 0; 2047 x 2049 x 513 38.4 -> 34.2 us,
+// 2048 x 4096 x 100 26.6 -> 27.9), then offsets that stay in registers and packed additions -9 to +6 % (median -1; 256 x
+// 4096 x 4096 51.8 -> 49.3, 301 x 303 x 305 7.0 -> 7.4): problems of 6 to 12 us gave up to 0.4 us for it.
 // CTA pairs: the rate the tensor pipe sustains under the power limit (six products of 2048 x 2048 x 1024 in 41 us:
 // 1.27 PFLOP/s, 1.6 in the loop).  Small problems: ~6 us of launch, first loads, last sums and stores.
 // Measured (graph replays), split copies by a pre-pass -> here: 1 x 1000 x 2048 35 -> 11.5 us, 300^3 12.9 -> 7.1, 1024^3
