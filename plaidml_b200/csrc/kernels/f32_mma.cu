@@ -25,7 +25,7 @@
 //
 // What bounds it: 64- and 128-wide tiles the loaders: per k-block of a 128-wide tile 64 KB of loads, 98 KB of stores and
 // 16,384 elements to cut, ~2300 cycles where the MMAs take 1536.  Copies of an earlier form (eight loader warps, 1024 x
-// 1024 x 4096, 90.6 us) with work left out: without the loads 71.4 us, without the stores 69.3, with two of the five MMAs
+// 1024 x 4096, 90.6 us) with work left out: without the loads 71.5 us, without the stores 69.3, with two of the five MMAs
 // 85.3.  Over 73 shapes 16 loader warps instead of eight took -12 to +5 % (median 0; 2047 x 2049 x 513 38.4 -> 34.2 us,
 // 2048 x 4096 x 100 26.6 -> 27.9), then offsets that stay in registers and packed additions -9 to +6 % (median -1; 256 x
 // 4096 x 4096 51.8 -> 49.3, 301 x 303 x 305 7.0 -> 7.4): problems of 6 to 12 us gave up to 0.4 us for it.
