@@ -26,9 +26,8 @@ struct ProductForm {
 // variables of a role must merge into one dimension; A and B each need a contiguous dimension, the output contiguous
 // columns (exchanging the sources transposes the product).  Every output element must be reached and every read in
 // range, since the tensor-core kernel tests neither.  More than 32768 multiply-adds: up to there the lean kernel adds the
-// terms one by one in f32, which small exact expectations rely on (the planner draws the same line for its GEMMs).  With
-// A transposed, general kernel -> tensor cores: 4096 x 512 x 512 23.4 ms -> 25 us, 128 x 64 x 64 295 -> 8 us (lean kernel
-// 32 us); error against 64 bits at 4096 terms 1.1e-6 -> 2.8e-7.
+// terms one by one in f32, which small exact expectations rely on (the planner draws the same line for its GEMMs).
+// Whether the product is also faster there: product_pays.
 inline bool product_form(const GenericParams& p, ProductForm* out) {
   if (p.agg != PMLB_AGG_SUM || p.combo != PMLB_COMBO_MUL || p.n_src != 2 || p.n_cons != 0 || p.has_init) return false;
   if (p.out.dtype != PMLB_F32 || p.src[0].dtype != PMLB_F32 || p.src[1].dtype != PMLB_F32) return false;
@@ -106,6 +105,22 @@ inline bool product_form(const GenericParams& p, ProductForm* out) {
     return true;
   }
   return false;
+}
+
+// Whether a contraction of product form goes to the tensor cores, `product_us` being the estimate for the tiles that would
+// be launched.  Fewer than 16 terms stay with the lean (else the general) kernel: there a plain f32 sum is as exact, one
+// k-block of the tensor-core kernel is 64 terms, and it was the slower one at every shape measured (4096 x 4096 outer
+// product 13 against 55 us, 512 x 512 x 8 terms 4.8 against 5.5).  From 16 on the estimates decide: batch entries and
+// single rows or columns cost a 128 x 64 tile each, whatever part of it exists.  The lean kernel takes 0.22 us per term
+// (its threads add term by term) or 6 multiply-adds per picosecond, the general one 2.3 us or 0.06 (B200, graph replays
+// of 137 shapes).  Lean against tensor cores: 65536 dot products of 64 terms 37 against 2209 us, 256 products of 32 x 32
+// x 32 10.7 against 11.3, 64 x 64 x 16 6.2 against 5.1, 4096 products of 64 x 64 x 64 236 against 168, 4096 x 512 x 512
+// with A transposed 23 ms (general), 945 (lean) against 23 us.
+inline bool product_pays(const ProductForm& f, bool lean, double product_us) {
+  if (f.k < 16) return false;
+  const double terms = static_cast<double>(f.k), macs = terms * f.m * f.n * f.batch;
+  const double other_us = 2.5 + (lean ? std::max(0.22 * terms, macs / 6e6) : std::max(2.3 * terms, macs / 6e4));
+  return product_us <= 0.95 * other_us;
 }
 
 // The lean kernel's form: see generic.cu.  Output dims are single variables without offset, everything is integral,

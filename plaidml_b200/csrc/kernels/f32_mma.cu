@@ -814,6 +814,8 @@ int resident_clusters(int dev, int split) {
   return known[dev][split];
 }
 
+constexpr long long kMaxTiles = 0x0fffffff;   // (times eight CTAs: the grid's limit)
+
 struct Choice {
   int bn = 0, split = 0;
   double cycles = 0;
@@ -828,7 +830,8 @@ Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_overri
   for (int bn = 64; bn <= (pairs ? 256 : 128); bn *= 2) {
     if (bn_override != 0 && bn != bn_override) continue;
     const int rows = bn == 256 ? 256 : 128;
-    const long long tiles = static_cast<long long>((m + rows - 1) / rows) * ((n + bn - 1) / bn) * batch;
+    const long long tiles = (m + rows - 1ll) / rows * ((n + bn - 1ll) / bn) * batch;
+    if (tiles > kMaxTiles) continue;
     for (int split = 1; split <= (bn == 256 ? 4 : 8); ++split) {
       if (split_override != 0 ? split != split_override : split > num_kb) continue;
       const int share = bn == 256 ? 2 * split : split;
@@ -875,7 +878,7 @@ F32MmaTiles f32_mma_tiles(const F32MmaShape& s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, s.tile_n, s.whole_k ? 1 : 0, !s.short_chains, dev, sms);
   F32MmaTiles t;
-  t.bn = c.bn, t.split = c.split;
+  t.bn = c.bn, t.split = c.split, t.us = c.cycles / 1900.0;
   return t;
 }
 
@@ -892,6 +895,7 @@ bool f32_mma_faster(const F32MmaShape& s, F32MmaTiles* tiles) {
   const Choice any = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, true, dev, sms);
   const double here = any.cycles / 1900.0 * (s.conv ? (any.bn == 256 ? 1.05 : 1.2) : 1.0);   // (gathering pixels costs more)
   *tiles = f32_mma_tiles(s);
+  if (any.bn == 0 || tiles->bn == 0) return false;
   const double tiles_m = (s.m + 127) / 128;
   auto prepass = [&](int bn, double block_us) {
     const double waves = std::max(1.0, tiles_m * ((s.n + bn - 1) / bn) * s.batch / sms);
@@ -936,7 +940,7 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   const int tile_rows = best_bn == 256 ? 256 : 128, share = best_bn == 256 ? 2 * p.split : p.split;
   const long long per_batch = static_cast<long long>((L.m + tile_rows - 1) / tile_rows) * p.tiles_n;
   const long long units = per_batch * L.batch;
-  if (units > 0x0fffffffll) {
+  if (units > kMaxTiles) {
     *err = "too many tiles";
     return PMLB_ERR_UNSUPPORTED;
   }

@@ -9,9 +9,11 @@
 
 namespace pmlb {
 
-// Tile width (64, 128: one CTA; 256: a CTA pair) and the number of CTAs (1..8) that share a tile's K range.
+// Tile width (64, 128: one CTA; 256: a CTA pair), the number of CTAs (1..8) that share a tile's K range, and the estimated
+// time.  bn 0: more tiles than a launch takes.
 struct F32MmaTiles {
   int bn = 64, split = 1;
+  double us = 0;
 };
 
 // C[b][i][j] = sum_k A(b, i, k) * B(b, k, j), everything fp32 in device memory.

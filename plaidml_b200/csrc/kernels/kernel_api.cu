@@ -1084,15 +1084,15 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
       if (!direct || !used[i]) p.loop_var[p.n_loop++] = i;
     }
   }
-  plan->f32_mma = pmlb::product_form(p, &plan->product);
-  plan->lean = !plan->f32_mma && pmlb::lean_form(p, &plan->lean_params);
-  if (plan->f32_mma) {
+  plan->lean = pmlb::lean_form(p, &plan->lean_params);
+  if (pmlb::product_form(p, &plan->product)) {
     const pmlb::ProductForm& f = plan->product;
     pmlb::F32MmaShape shape;
     shape.m = static_cast<int>(f.m), shape.n = static_cast<int>(f.n), shape.k = static_cast<int>(f.k), shape.batch = static_cast<int>(f.batch);
     shape.aligned_in = (f.ak == 1 ? f.am : f.ak) % 4 == 0 && (f.bk == 1 ? f.bn : f.bk) % 4 == 0;
     shape.short_chains = true;
     plan->f32_tiles = pmlb::f32_mma_tiles(shape);
+    plan->f32_mma = plan->f32_tiles.bn != 0 && pmlb::product_pays(f, plan->lean, plan->f32_tiles.us);
   }
   pmlb_status st = alloc_plan_memory(plan, 0, plan->f32_mma);
   if (st != PMLB_OK) {

@@ -3,8 +3,12 @@
 // check ("ok <name>" / "FAIL <name> ...") and exits non-zero on any failure.
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
+#include <map>
 #include <random>
+#include <string>
 
+#include "contract_route.h"
 #include "conv_route.h"
 #include "tc_gemm.cuh"
 
@@ -30,6 +34,42 @@ static pmlb_conv_desc conv(int n, int h, int w, int c, int r, int s, int k, int 
   d.q = (w + 2 * pad - s) / stride + 1;
   d.epilogue = epi;
   return d;
+}
+
+// out[c] += a[a] * b[b], one letter per index variable, everything dense f32.
+static pmlb::GenericParams contraction(const char* a, const char* b, const char* c, std::map<char, long long> ext) {
+  pmlb::GenericParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.agg = PMLB_AGG_SUM;
+  p.combo = PMLB_COMBO_MUL;
+  p.n_src = 2;
+  p.direct = 1;
+  p.out_elems = 1;
+  std::map<char, int> var;
+  for (const auto& e : ext) {
+    var[e.first] = p.n_idx;
+    p.range[p.n_idx++] = e.second;
+  }
+  auto fill = [&](pmlb::GAccess* t, const std::string& dims) {
+    t->dtype = PMLB_F32;
+    t->rank = static_cast<int>(dims.size());
+    long long stride = 1;
+    for (int d = t->rank - 1; d >= 0; --d) {
+      t->sizes[d] = ext[dims[d]];
+      t->strides[d] = stride;
+      stride *= t->sizes[d];
+      t->den[d] = 1;
+      t->coef[d][var[dims[d]]] = 1;
+    }
+  };
+  fill(&p.out, c);
+  fill(&p.src[0], a);
+  fill(&p.src[1], b);
+  for (int d = 0; d < p.out.rank; ++d) {
+    p.out_var[d] = var[c[d]];
+    p.out_elems *= p.out.sizes[d];
+  }
+  return p;
 }
 
 int main() {
@@ -76,6 +116,31 @@ int main() {
           "7x7/2 pad 3 -> 4x4 taps, 115 rows of 128 pixels, 928 pixels per tile");
     const pmlb::S2dShape e = pmlb::conv_s2d_shape(conv(2, 20, 22, 2, 4, 2, 16, 2, 1));
     check(e.pe_h == 2 && e.dh == 1 && e.r2 == 3 && e.s2 == 2 && e.wp % 32 == 0 && e.stage_px % 32 == 0, "even filter, odd padding");
+  }
+  // contractions: which are matrix products, and which of these pay on the tensor cores (us: the tiles' estimate)
+  {
+    pmlb::ProductForm f;
+    pmlb::LeanParams l;
+    auto form = [&](const pmlb::GenericParams& p, long long b, long long m, long long n, long long k) {
+      return pmlb::product_form(p, &f) && pmlb::lean_form(p, &l) && f.batch == b && f.m == m && f.n == n && f.k == k;
+    };
+    check(form(contraction("km", "kn", "mn", {{'k', 4096}, {'m', 512}, {'n', 512}}), 1, 512, 512, 4096) && f.am == 1 && f.ak == 512 &&
+              pmlb::product_pays(f, true, 24.0),
+          "weight gradient: product");
+    check(form(contraction("ij", "ij", "ij", {{'i', 1024}, {'j', 1024}}), 1 << 20, 1, 1, 1) && !pmlb::product_pays(f, true, 1.0),
+          "element-wise product: strided");
+    check(form(contraction("yc", "c", "yc", {{'c', 128}, {'y', 100352}}), 128, 100352, 1, 1) && !pmlb::product_pays(f, true, 1.0),
+          "scale per channel: strided");
+    check(form(contraction("i", "j", "ij", {{'i', 4096}, {'j', 4096}}), 1, 4096, 4096, 1) && !pmlb::product_pays(f, true, 1.0),
+          "outer product: strided");
+    check(form(contraction("ik", "ik", "i", {{'i', 65536}, {'k', 64}}), 65536, 1, 1, 64) && !pmlb::product_pays(f, true, 2400.0) &&
+              pmlb::product_pays(f, true, 10.0),
+          "many short dot products: strided unless the estimate is small");
+    check(form(contraction("km", "kn", "mn", {{'k', 15}, {'m', 512}, {'n', 512}}), 1, 512, 512, 15) && !pmlb::product_pays(f, false, 1.0),
+          "fifteen terms: never on the tensor cores");
+    check(form(contraction("km", "kn", "mn", {{'k', 16}, {'m', 128}, {'n', 128}}), 1, 128, 128, 16) && pmlb::product_pays(f, true, 5.5) &&
+              !pmlb::product_pays(f, true, 6.0),
+          "sixteen terms: by the estimate");
   }
   return failures == 0 ? 0 : 1;
 }

@@ -545,6 +545,42 @@ def test_products_in_any_order_of_dims(seed):
     assert np.linalg.norm(out - want) / norm <= max(1.5 * np.linalg.norm(ref - want) / norm, 2.0 ** -20)
 
 
+@pytest.mark.parametrize("a,b,c,ext", [
+    ("ij", "ij", "ij", {"i": 211, "j": 307}),                # all batch dims
+    ("yc", "c", "yc", {"y": 25089, "c": 24}),                # a scale per channel
+    ("ij", "i", "ij", {"i": 130, "j": 1001}),
+    ("i", "j", "ij", {"i": 513, "j": 770}),                  # no terms
+    ("km", "kn", "mn", {"m": 130, "n": 70, "k": 15}),        # too few terms
+    ("ik", "ik", "i", {"i": 5000, "k": 40}),                 # one dot product per batch entry
+    ("bkm", "bkn", "bmn", {"b": 3000, "m": 4, "n": 3, "k": 20}),
+])
+def test_products_that_leave_their_tiles_empty_add_term_by_term(a, b, c, ext):
+    g = rng(7250 + len(ext))
+    var = {v: i for i, v in enumerate(ext)}
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, len(ext), 2
+    for v, i in var.items():
+        d.range[i] = ext[v]
+    acc = lambda dims: K.make_access(K.F32, [ext[v] for v in dims], [{var[v]: 1} for v in dims])
+    d.out, d.src[0], d.src[1] = acc(c), acc(a), acc(b)
+    x, y = (g.standard_normal([ext[v] for v in dims]).astype(np.float32) for dims in (a, b))
+    out, ref = run_contract(d, [x, y], tuple(ext[v] for v in c), K.F32)
+    np.testing.assert_array_equal(out, ref)
+
+
+def test_more_products_than_a_launch_takes_tiles():
+    n = (1 << 28) + 3
+    x, y = (torch.rand(n, device="cuda") - 0.5 for _ in range(2))
+    out = torch.empty(n, device="cuda")
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 1, 2
+    d.range[0] = n
+    d.out = K.make_access(K.F32, [n], [{0: 1}])
+    d.src[0] = d.src[1] = K.make_access(K.F32, [n], [{0: 1}])
+    K.Plan("contract", d).contract([ptr(x), ptr(y)], ptr(out))
+    assert torch.equal(out, x * y)
+
+
 def test_product_that_does_not_cover_its_output_or_reads_out_of_range_stays_exact():
     # a range shorter than the output dim leaves the identity there; one longer than an operand's dim skips terms
     g = rng(7300)
