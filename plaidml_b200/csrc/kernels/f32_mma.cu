@@ -36,7 +36,7 @@
 // 28 x 128 -> 128, 3x3 25.5 -> 20.0, 32 x 7 x 7 x 512 -> 512, 3x3 63 -> 45 (pairs, K in parts), 1 x 7 x 7 x 512 61 -> 15.
 // Walking several tiles per CTA with the stores behind the next tile's loads was slower (1024^3 21.2 us against 19.2).
 //
-// inf / NaN: x - h is NaN for them, so only hh is right; a sum whose hh part is not finite drops its small part.
+// inf / NaN: h is inf / NaN, x - h is NaN, so only hh is right; a sum whose hh part is not finite drops its small part.
 #include "f32_mma.h"
 
 #include <cuda_bf16.h>
@@ -127,6 +127,14 @@ __device__ __forceinline__ uint32_t upper_halves(float lo, float hi) {
   return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
 }
 
+// Two floats cut to bf16, x in the lower half.  Not upper_halves: NaN stays NaN also where its payload is in the bits that
+// are cut off.
+__device__ __forceinline__ uint32_t cut_to_bf16(float x, float y) {
+  uint32_t r;
+  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+  return r;
+}
+
 // (a, b) + (c, d) in one instruction.
 __device__ __forceinline__ float2 add2(float a, float b, float c, float d) {
   float2 r;
@@ -158,7 +166,7 @@ __device__ __forceinline__ void st_shared_b32(uint32_t addr, uint32_t x) {
 
 // Cuts consecutive elements into the three parts and stores 8 (4) bytes of each.
 __device__ __forceinline__ void store_parts(uint32_t addr, uint32_t part_bytes, const float (&v)[4]) {
-  st_shared_v2(addr, upper_halves(v[0], v[1]), upper_halves(v[2], v[3]));
+  st_shared_v2(addr, cut_to_bf16(v[0], v[1]), cut_to_bf16(v[2], v[3]));
   const float2 m0 = rest_of(v[0], v[1]), m1 = rest_of(v[2], v[3]);
   st_shared_v2(addr + part_bytes, upper_halves(m0.x, m0.y), upper_halves(m1.x, m1.y));
   const float2 l0 = rest_of(m0.x, m0.y), l1 = rest_of(m1.x, m1.y);
@@ -166,7 +174,7 @@ __device__ __forceinline__ void store_parts(uint32_t addr, uint32_t part_bytes, 
 }
 
 __device__ __forceinline__ void store_parts(uint32_t addr, uint32_t part_bytes, const float (&v)[2]) {
-  st_shared_b32(addr, upper_halves(v[0], v[1]));
+  st_shared_b32(addr, cut_to_bf16(v[0], v[1]));
   const float2 m = rest_of(v[0], v[1]);
   st_shared_b32(addr + part_bytes, upper_halves(m.x, m.y));
   const float2 l = rest_of(m.x, m.y);

@@ -474,6 +474,32 @@ def test_f32_split_operands_keep_infinities_and_nan():
     assert max_rel(got[rows], want[rows]) < 1e-6
 
 
+@pytest.mark.parametrize("m,n,k,tile_n", [
+    (130, 70, 300, 64),
+    (130, 140, 300, 128),
+    (60, 70, 2000, 0),          # K shared by a cluster
+    (2047, 2049, 513, 0),       # CTA pairs
+])
+def test_f32_split_operands_keep_every_nan(m, n, k, tile_n):
+    # NaN whose payload is in the 16 bits that the first part of an operand does not hold, of both signs, and others
+    g = rng(3300 + k)
+    a = g.uniform(0.5, 1, size=(1, m, k)).astype(np.float32)
+    b = g.uniform(0.5, 1, size=(1, k, n)).astype(np.float32)
+    clean = run_gemm(K.F32, K.F32, dev(a), dev(b), m, n, k, 1, False, tile_n=tile_n)[0].cpu().numpy()[0]
+    patterns = np.array([0x7f800001, 0xff800001, 0x7f80ffff, 0xff808000, 0x7fc00000, 0xffffffff], dtype=np.uint32)
+    rows, cols = [0, 7, 31, 32, 58, m - 1], [1, 2, 33, 63, 64, n - 1]
+    for r, c, bits in zip(rows, cols, patterns):
+        a.view(np.uint32)[0, r, int(g.integers(0, k))] = bits
+        b.view(np.uint32)[0, int(g.integers(0, k)), c] = bits
+    bias = dev(np.zeros(n, dtype=np.float32))
+    for epi in (0, K.EPI_BIAS | K.EPI_RELU):
+        got = run_gemm(K.F32, K.F32, dev(a), dev(b), m, n, k, 1, False, tile_n=tile_n, epilogue=epi, bias=bias)[0].cpu().numpy()[0]
+        want = clean.copy()
+        want[rows, :] = np.nan
+        want[:, cols] = np.nan
+        np.testing.assert_array_equal(got, want)
+
+
 # --- CTA pairs (two CTAs per 256 x 256 tile) -----------------------------------------------------
 
 @pytest.mark.parametrize("b_is_nk", [True, False], ids=["B[n][k]", "B[k][n]"])
