@@ -1,6 +1,12 @@
 // fp32 products on the tensor cores: every operand element x is cut into three bf16 parts x = h + m + l of 8
-// significant bits each (exact for 24 bits), and a product is the six part products that are above 2^-24 of it:
-// hh + (hm + mh + hl + lh + mm).  bf16 MMAs run at twice the TF32 rate, so six of them cost what three TF32 products
+// significant bits each, h towards zero (the largest finite values stay finite), m to nearest, l what is left (exact for
+// 24 bits, |m| < 2^-7 and |l| <= 2^-16 of x's power of two, l of either sign), and a product is six of the nine part
+// products: hh + (hm + mh + hl + lh + mm).  The two next ones, ml and lm, are 2^-22 of the product at most and cancel
+// over a sum: with m cut towards zero as well they reached 2^-21 and all had the product's sign (4e-8 of every sum of
+// positive terms).  Error of a single product against 64 bits, in norm: 3.0e-8 (5.1e-8 with m cut; plain f32 2.5e-8,
+// three TF32 products 6.6e-8), of sums of 8 to 4096 terms 0.6 to 0.2 times that of plain f32 sums.  bf16 parts end at
+// 2^-133: operands below 2^-110 lose what lies under 2^-134 (2^-16 of themselves at 2^-118).
+// bf16 MMAs run at twice the TF32 rate, so six of them cost what three TF32 products
 // cost, but the parts keep all 24 bits (two TF32 parts keep 22), occupy 6 bytes of shared memory per element instead
 // of 8, and bf16 operands may be MN-major, so a [k][n] B or a transposed A needs no transposition.
 //
@@ -14,7 +20,7 @@
 //                in shared memory, so one MMA of width 2 BN does hh and hm with one read of A.
 //   warps 16..23 after every kFlushBlocks k-blocks (256 terms) they add both accumulators to sums in registers with
 //                round-to-nearest while the issuer goes on with the other accumulator pair: chains of 16 MMAs instead
-//                of k / 8.  Error against 64 bits at 2048 terms: 2.3e-7, three TF32 products in one chain 1.4e-5.
+//                of k / 8.  Error against 64 bits at 2048 terms: 2.0e-7, three TF32 products in one chain 1.4e-5.
 //   all warps    the sums go through shared memory (free by then) to row-contiguous 16-byte stores with the epilogue.
 //
 // Few tiles and a long K: `split` CTAs of a cluster share a tile, each a contiguous run of k-blocks; every CTA then
@@ -135,6 +141,12 @@ __device__ __forceinline__ uint32_t cut_to_bf16(float x, float y) {
   return r;
 }
 
+__device__ __forceinline__ uint32_t round_to_bf16(float x, float y) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+  return r;
+}
+
 // (a, b) + (c, d) in one instruction.
 __device__ __forceinline__ float2 add2(float a, float b, float c, float d) {
   float2 r;
@@ -143,6 +155,20 @@ __device__ __forceinline__ float2 add2(float a, float b, float c, float d) {
       "mov.b64 x, {%2, %3};\n\t"
       "mov.b64 y, {%4, %5};\n\t"
       "add.rn.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t"
+      "}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
+}
+
+__device__ __forceinline__ float2 sub2(float a, float b, float c, float d) {
+  float2 r;
+  asm("{\n\t"
+      ".reg .b64 x, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "sub.rn.f32x2 x, x, y;\n\t"
       "mov.b64 {%0, %1}, x;\n\t"
       "}"
       : "=f"(r.x), "=f"(r.y)
@@ -164,21 +190,33 @@ __device__ __forceinline__ void st_shared_b32(uint32_t addr, uint32_t x) {
   asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");
 }
 
-// Cuts consecutive elements into the three parts and stores 8 (4) bytes of each.
+// Cuts two elements into the three parts.  One conversion per part, as cheap as taking upper halves (1024^3 17.7 us both).
+struct Parts {
+  uint32_t h, m, l;
+};
+__device__ __forceinline__ Parts cut(float x, float y) {
+  Parts c;
+  c.h = cut_to_bf16(x, y);
+  const float2 r = rest_of(x, y);
+  c.m = round_to_bf16(r.x, r.y);
+  const float2 l = sub2(r.x, r.y, __uint_as_float(c.m << 16), __uint_as_float(c.m & 0xffff0000u));
+  c.l = upper_halves(l.x, l.y);
+  return c;
+}
+
+// Stores 8 (4) bytes of each part of consecutive elements.
 __device__ __forceinline__ void store_parts(uint32_t addr, uint32_t part_bytes, const float (&v)[4]) {
-  st_shared_v2(addr, cut_to_bf16(v[0], v[1]), cut_to_bf16(v[2], v[3]));
-  const float2 m0 = rest_of(v[0], v[1]), m1 = rest_of(v[2], v[3]);
-  st_shared_v2(addr + part_bytes, upper_halves(m0.x, m0.y), upper_halves(m1.x, m1.y));
-  const float2 l0 = rest_of(m0.x, m0.y), l1 = rest_of(m1.x, m1.y);
-  st_shared_v2(addr + 2 * part_bytes, upper_halves(l0.x, l0.y), upper_halves(l1.x, l1.y));
+  const Parts a = cut(v[0], v[1]), b = cut(v[2], v[3]);
+  st_shared_v2(addr, a.h, b.h);
+  st_shared_v2(addr + part_bytes, a.m, b.m);
+  st_shared_v2(addr + 2 * part_bytes, a.l, b.l);
 }
 
 __device__ __forceinline__ void store_parts(uint32_t addr, uint32_t part_bytes, const float (&v)[2]) {
-  st_shared_b32(addr, cut_to_bf16(v[0], v[1]));
-  const float2 m = rest_of(v[0], v[1]);
-  st_shared_b32(addr + part_bytes, upper_halves(m.x, m.y));
-  const float2 l = rest_of(m.x, m.y);
-  st_shared_b32(addr + 2 * part_bytes, upper_halves(l.x, l.y));
+  const Parts a = cut(v[0], v[1]);
+  st_shared_b32(addr, a.h);
+  st_shared_b32(addr + part_bytes, a.m);
+  st_shared_b32(addr + 2 * part_bytes, a.l);
 }
 
 // One loader thread's share of an operand tile of ROWS rows (m or n) x 64 terms.  `origin`: row 0 of the tile, term 0

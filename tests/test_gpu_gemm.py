@@ -448,7 +448,7 @@ def test_f32_operands_split_in_the_kernel(m, n, k, b_is_nk, tile_n, offset):
                           tile_n=tile_n)
     assert plan.scratch_bytes == 256    # the status word: no split copies
     ref = np.maximum(oracle.gemm_f32_acc64(a, b, b_is_nk) + bias, 0)
-    # products keep 24 bits (2^-24 each); a chain of 16 (pairs: k / 16) truncating additions of at most 2^-23 of the
+    # products are within 2^-22 of theirs; a chain of 16 (pairs: k / 16) truncating additions of at most 2^-23 of the
     # largest partial sum, which a random walk leaves below twice the largest result
     chain = 16 if m < 2000 else (k + 15) // 16
     assert max_rel(c.cpu().numpy(), ref) < (2 * chain + 8) * 2.0 ** -23
@@ -472,6 +472,40 @@ def test_f32_split_operands_keep_infinities_and_nan():
     assert got[11, 2] == np.inf
     rows = [r for r in range(m) if r not in (3, 5, 9, 11)]
     assert max_rel(got[rows], want[rows]) < 1e-6
+
+
+@pytest.mark.parametrize("x,y", [
+    (1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -7 - 2.0 ** -23),       # everything below the first part set
+    (1 + 2.0 ** -7 - 2.0 ** -16, 1 + 2.0 ** -7 - 2.0 ** -16),       # a middle part that is rounded by half its last place
+    (1 + 2.0 ** -7 - 3 * 2.0 ** -16, -(1 + 2.0 ** -7 - 2.0 ** -23)),
+    (2 - 2.0 ** -23, 2 - 2.0 ** -23),
+    (-3.4028234663852886e38, 2.0 ** -64),                           # the lowest finite value stays finite
+    (2.0 ** -109 * (2 - 2.0 ** -23), 1 + 2.0 ** -7 - 2.0 ** -23),   # the last binades whose last part is whole
+])
+@pytest.mark.parametrize("tile_n", [64, 128])
+def test_f32_part_products_of_the_worst_mantissas(x, y, tile_n):
+    # 64 equal terms: one k-block
+    m, n, k = 128, 128, 64
+    a, b = np.full((1, m, k), x, dtype=np.float32), np.full((1, k, n), y, dtype=np.float32)
+    assert a[0, 0, 0] == x and b[0, 0, 0] == y
+    c, _, plan = run_gemm(K.F32, K.F32, dev(a), dev(b), m, n, k, 1, False, tile_n=tile_n)
+    assert plan.scratch_bytes == 256
+    # the two part products left out are 2^-22 together; the chain's large sums are whole multiples of h h (exact up to 64
+    # of them), the small ones are 2^-6 of it and lose 16 times 2^-23 of themselves, and the result is rounded
+    assert np.max(np.abs(c.cpu().numpy() / (64 * x * y) - 1)) <= 2.0 ** -22 + 2.0 ** -24 + 2.0 ** -25
+
+
+def test_f32_part_products_of_short_sums_and_small_operands():
+    g = rng(3250)
+    m = n = 512
+    for k, scale, bound in ((1, 1.0, 2.0 ** -24.5),       # rounding a product is 2^-25.3 in norm, the parts left out 2^-25.7
+                            (8, 1.0, 2.0 ** -24),
+                            (8, 2.0 ** -118, 2.0 ** -14)):  # up to 2^-134 lost of every operand of about 2^-119
+        a = (g.uniform(-1, 1, size=(1, m, k)) * scale).astype(np.float32)
+        b = g.uniform(-1, 1, size=(1, k, n)).astype(np.float32)
+        c = run_gemm(K.F32, K.F32, dev(a), dev(b), m, n, k, 1, False)[0].cpu().numpy()[0].astype(np.float64)
+        want = a[0].astype(np.float64) @ b[0].astype(np.float64)
+        assert np.linalg.norm(c - want) <= bound * np.linalg.norm(want), (k, scale)
 
 
 @pytest.mark.parametrize("m,n,k,tile_n", [
