@@ -456,7 +456,15 @@ __device__ __forceinline__ void finish(const F32MmaParams& p, int batch, int i, 
   }
 }
 
-template <int BN, int AL, int BL, bool VEC>
+// Contractions come from a kernel that adds plain f32 products, and keep its results where three bf16 parts cannot
+// stand for an operand: infinity times a subnormal below 2^-133 (whose parts are 0: NaN), and rows of operands below
+// 2^-110.  Such results are recognised by what they are (NaN, or not zero and below 2^-100) and added again, term by
+// term, by the thread that stored them, after everything else.  The others pay the comparison: 0.1 to 0.3 us of a launch
+// (64 x 64 x 64 4.65 -> 4.87 us, 1000 x 999 x 301 11.7 -> 11.8, 512 x 512 x 4096 21.5 -> 21.4).
+__device__ __forceinline__ bool parts_fail(float v) { return !(fabsf(v) >= 0x1p-100f) & (v != 0.f); }
+
+// CONTRACT: the launch of a contraction.
+template <int BN, int AL, int BL, bool VEC, bool CONTRACT>
 __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_constant__ F32MmaParams p) {
   using Cfg = F32Cfg<BN>;
   constexpr bool PAIR = Cfg::kPair;
@@ -752,6 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
   }
   const bool failed = abort_flag[0] != 0;
   grid_dependency_wait();   // (long past for the loaders; the other warps have not touched global memory yet)
+  bool again = false;
   if (!failed && warp < kIssuerWarp) {
     constexpr int kPieces = BN / 4;                 // 16-byte pieces per row
     const int strip = (128 + strips - 1) / strips;
@@ -787,6 +796,10 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
         if (piece % 32 == 0 && mine && i < p.m) atomic_max_f32(p.rowmax + static_cast<long long>(batch) * p.m + i, best);
         if (p.out == nullptr) continue;
       }
+      if constexpr (CONTRACT) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) again |= parts_fail(o[e]);
+      }
       if (valid > 0) finish(p, batch, i, j, o, valid);
     }
   }
@@ -810,6 +823,40 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
       tmem_dealloc(*tmem_slot, 512);
     }
   }
+  if (CONTRACT && __builtin_expect(again, 0)) {
+    constexpr int kPieces = BN / 4;
+    const int strip = (128 + strips - 1) / strips;
+    const int strip_begin = strips > 1 ? rank * strip : 0;
+    const int strip_end = min(128, strip_begin + strip);
+    const long long step_a = AL == kRowsMn ? p.lda : 1, step_b = BL == kRowsMn ? p.ldb : 1, step_j = BL == kRowsMn ? 1 : p.ldb;
+#pragma unroll 1
+    for (int t = threadIdx.x; t < strip * kPieces; t += kIssuerWarp * 32) {
+      const int i = m0 + strip_begin + t / kPieces, j = n0 + t % kPieces * 4;
+      if (strip_begin + t / kPieces >= strip_end || i >= p.m) break;   // (rows only grow)
+      const int cols = min(4, p.n - j);
+      float* dst = p.out + batch * p.out_batch + static_cast<long long>(i) * p.ldc + j;
+      bool any = false;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) any |= e < cols && parts_fail(dst[e]);
+      if (!any) continue;
+      const float* a = p.a + batch * p.a_batch + (AL == kRowsMn ? static_cast<long long>(i) : i * p.lda);
+      const float* b = p.b + batch * p.b_batch + j * step_j;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      bool number = true;   // (NaN stays)
+#pragma unroll 1
+      for (int k = 0; k < p.k && number; ++k) {
+        const float x = __ldg(a);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] = __fadd_rn(sum[e], __fmul_rn(x, __ldg(b + (e < cols ? e : 0) * step_j)));
+        number = sum[0] == sum[0] || sum[1] == sum[1] || sum[2] == sum[2] || sum[3] == sum[3];
+        a += step_a, b += step_b;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (e < cols && parts_fail(dst[e])) dst[e] = sum[e];
+      }
+    }
+  }
 }
 
 template <class In>
@@ -821,16 +868,16 @@ __global__ void __launch_bounds__(256) filter_to_f32_kernel(const In* in, float*
 using KernelPtr = void (*)(const F32MmaParams);
 
 // The shared-memory limit is an attribute per device.
-template <int BN, int AL, int BL, bool VEC>
+template <int BN, int AL, int BL, bool VEC, bool CONTRACT = false>
 KernelPtr instance(int dev) {
   static std::atomic<uint64_t> done{0};
   const uint64_t bit = 1ull << (dev & 63);
   if (dev >= 64 || (done.load(std::memory_order_acquire) & bit) == 0) {
-    if (cudaFuncSetAttribute(f32_mma_kernel<BN, AL, BL, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Cfg<BN>::kSmem) == cudaSuccess) {
+    if (cudaFuncSetAttribute(f32_mma_kernel<BN, AL, BL, VEC, CONTRACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, F32Cfg<BN>::kSmem) == cudaSuccess) {
       done.fetch_or(bit, std::memory_order_release);
     }
   }
-  return f32_mma_kernel<BN, AL, BL, VEC>;
+  return f32_mma_kernel<BN, AL, BL, VEC, CONTRACT>;
 }
 
 // Clusters of `split` CTAs that the device holds at once (a GPC holds whole clusters only).
@@ -896,15 +943,24 @@ Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_overri
   return best;
 }
 
-template <int BN>
-KernelPtr choose(int al, int bl, bool vec, int dev) {
-  if (al == kRowsConv) return vec ? instance<BN, kRowsConv, kRowsMn, true>(dev) : instance<BN, kRowsConv, kRowsMn, false>(dev);
-  if (vec) {
-    if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, true>(dev) : instance<BN, kRowsK, kRowsMn, true>(dev);
-    return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, true>(dev) : instance<BN, kRowsMn, kRowsMn, true>(dev);
-  }
-  if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, false>(dev) : instance<BN, kRowsK, kRowsMn, false>(dev);
-  return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, false>(dev) : instance<BN, kRowsMn, kRowsMn, false>(dev);
+// A has its columns contiguous in contractions only.
+template <int BN, bool VEC>
+KernelPtr choose(int al, int bl, int dev) {
+  if (al == kRowsConv) return instance<BN, kRowsConv, kRowsMn, VEC>(dev);
+  return bl == kRowsK ? instance<BN, kRowsK, kRowsK, VEC>(dev) : instance<BN, kRowsK, kRowsMn, VEC>(dev);
+}
+
+template <int BN, bool VEC>
+KernelPtr choose_contraction(int al, int bl, int dev) {
+  if (al == kRowsK) return bl == kRowsK ? instance<BN, kRowsK, kRowsK, VEC, true>(dev) : instance<BN, kRowsK, kRowsMn, VEC, true>(dev);
+  return bl == kRowsK ? instance<BN, kRowsMn, kRowsK, VEC, true>(dev) : instance<BN, kRowsMn, kRowsMn, VEC, true>(dev);
+}
+
+template <bool VEC>
+KernelPtr choose(int bn, bool contraction, int al, int bl, int dev) {
+  if (contraction) return bn == 128 ? choose_contraction<128, VEC>(al, bl, dev) : choose_contraction<64, VEC>(al, bl, dev);
+  if (bn == 256) return choose<256, VEC>(al, bl, dev);
+  return bn == 128 ? choose<128, VEC>(al, bl, dev) : choose<64, VEC>(al, bl, dev);
 }
 
 }  // namespace
@@ -993,7 +1049,11 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   p.tiles_per_batch = static_cast<int>(per_batch);
   const long long grid = units * share;
   const int bl = L.b_mn ? kRowsMn : kRowsK;
-  const KernelPtr kernel = best_bn == 256 ? choose<256>(al, bl, vec, dev) : (best_bn == 128 ? choose<128>(al, bl, vec, dev) : choose<64>(al, bl, vec, dev));
+  if (L.contraction ? best_bn == 256 : L.a_mn) {
+    *err = "no such tiles";
+    return PMLB_ERR_UNSUPPORTED;
+  }
+  const KernelPtr kernel = vec ? choose<true>(best_bn, L.contraction, al, bl, dev) : choose<false>(best_bn, L.contraction, al, bl, dev);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kThreads);

@@ -34,6 +34,7 @@ struct F32MmaLaunch {
   const float* residual = nullptr;
   long long ldr = 0, res_batch = 0;
   float* rowmax = nullptr;          // f32[batch * m], filled with -inf by the caller
+  bool contraction = false;         // tiles without pairs; results that the parts cannot give are added again (f32_mma.cu)
   int* status = nullptr;            // device word that receives a non-zero code if a wait times out
   F32MmaTiles tiles;
 };

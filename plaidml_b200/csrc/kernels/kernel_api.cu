@@ -1122,6 +1122,7 @@ pmlb_status pmlb_contract_invoke(pmlb_plan* plan, void* stream, const void* src0
     L.b_mn = f.k > 1 && f.bk != 1;
     L.ldb = L.b_mn ? f.bk : f.bn;
     L.out = static_cast<float*>(outp), L.ldc = f.cm, L.out_batch = f.cb;
+    L.contraction = true;
     L.status = plan->status;
     L.tiles = plan->f32_tiles;
     std::string err;

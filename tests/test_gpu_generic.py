@@ -581,6 +581,35 @@ def test_more_products_than_a_launch_takes_tiles():
     assert torch.equal(out, x * y)
 
 
+@pytest.mark.parametrize("a,b,c,m,n,k", [("km", "kn", "mn", 130, 70, 64), ("km", "kn", "mn", 40, 36, 2000), ("mk", "nk", "nm", 150, 40, 48),
+                                         ("km", "nk", "mn", 129, 131, 130), ("mk", "kn", "mn", 300, 200, 515)])
+def test_products_of_infinite_and_of_tiny_operands(a, b, c, m, n, k):
+    ext = {"m": m, "n": n, "k": k}
+    var = {v: i for i, v in enumerate(ext)}
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 3, 2
+    for v, i in var.items():
+        d.range[i] = ext[v]
+    acc = lambda dims: K.make_access(K.F32, [ext[v] for v in dims], [{var[v]: 1} for v in dims])
+    d.out, d.src[0], d.src[1] = acc(c), acc(a), acc(b)
+    g = rng(7400 + k)
+    x, y = g.uniform(0.5, 1, (m, k)).astype(np.float32), g.uniform(0.5, 1, (k, n)).astype(np.float32)
+    x[3, 5], x[7, k - 1], x[9, 2] = np.inf, -np.inf, np.nan
+    y[5, 4], y[5, 6], y[k - 1, 8] = 2.0 ** -140, 0.0, -(2.0 ** -149)     # inf times these: inf, NaN, +inf
+    x[11] *= 2.0 ** -120                                                  # rows whose parts would end above their last bits
+    x[13] *= 2.0 ** -130
+    x[15] = 0
+    out, _ = run_contract(d, [np.ascontiguousarray(v) for v in (x if a == "mk" else x.T, y if b == "kn" else y.T)], tuple(ext[v] for v in c), K.F32)
+    got = out if c == "mn" else out.T
+    with np.errstate(invalid="ignore"):
+        want = x.astype(np.float64) @ y.astype(np.float64)
+        off = np.abs(got - want)
+    np.testing.assert_array_equal(np.where(np.isfinite(got), 0, got), np.where(np.isfinite(want), 0, want))
+    fine = np.isfinite(want)
+    # plain f32 sums: k roundings of at most 2^-24 of a sum of positive terms, and 2^-150 where a term is subnormal
+    assert np.all(off[fine] <= k * (2.0 ** -24 * np.abs(want[fine]) + 2.0 ** -150))
+
+
 def test_product_that_does_not_cover_its_output_or_reads_out_of_range_stays_exact():
     # a range shorter than the output dim leaves the identity there; one longer than an operand's dim skips terms
     g = rng(7300)
