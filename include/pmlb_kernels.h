@@ -98,7 +98,8 @@ pmlb_status pmlb_plan_share_status(pmlb_plan* plan, int* device_word);
 
 /* Name of the kernel family a plan resolved to ("tc_gemm", "tc_conv", "row_reduce", ...). */
 const char* pmlb_plan_kind(const pmlb_plan* plan);
-/* Parts the K range of a GEMM plan is split into (1 = a single pass). */
+/* Parts the K range of a GEMM plan is split into (1 = a single pass): by two passes for 8/16-bit inputs, among the CTAs of
+ * a cluster within one launch for fp32. */
 int pmlb_plan_split_k(const pmlb_plan* plan);
 /* Test hook for the bounded waits of the tensor-core kernel (no counterpart in the reference).  Every
  * device-side wait (on an operand stage, an accumulator, a residual row) gives up after a wall-clock limit,
@@ -173,7 +174,13 @@ typedef struct {
  * single pass, so a problem that is split at one size and not at another (the tile count decides) can
  * differ in the last bits between the two.  NO_SPLIT_K keeps one pass; SPLIT_K splits whenever the
  * k-blocks divide evenly, whatever the tile count (for testing); PMLB_SPLIT_K=0 in the environment turns
- * the library's own choice off for a whole process. */
+ * the library's own choice off for a whole process.
+ * fp32: tile kind, K split and kernel all follow the shape, and the order of the additions with them, so the last bits
+ * of a row can differ between problems of few and of many rows.  NO_SPLIT_K fixes them (one kernel, no split, tiles that
+ * add in one order): a row's sums are then the same whatever m and batch are, at up to 1.35 times the time of the kernel
+ * that would be chosen without a split, or twice where that is the TF32 pre-pass.  PMLB_SPLIT_K=0 does so for fp32 GEMMs
+ * and for fp32 convolutions on whole groups of four channels (the others add in one order anyway), and keeps contractions
+ * (pmlb_contract_dispatch) with the kernels that add term by term. */
 #define PMLB_GEMM_NO_SPLIT_K 64
 #define PMLB_GEMM_SPLIT_K 128
 

@@ -1148,9 +1148,10 @@ class Planner {
         if (pmlb_plan_split_k(plan) > 1) os << " splitk=" << pmlb_plan_split_k(plan);
         st.detail = os.str();
         // (+ the TF32 split of both operands where the plan holds room for it, + the row-max fill, + the combining pass
-        // of a split K range)
-        const bool split = pd.gemm.in_dtype == PMLB_F32 && pmlb_plan_scratch_bytes(plan) > 256;
-        st.launches = 1 + (split ? 1 : 0) + (pd.rowmax >= 0 ? 1 : 0) + (pmlb_plan_split_k(plan) > 1 ? 1 : 0);
+        // of a split K range; fp32 splits K within its one launch)
+        const bool f32 = pd.gemm.in_dtype == PMLB_F32;
+        const bool second = f32 ? pmlb_plan_scratch_bytes(plan) > 256 : pmlb_plan_split_k(plan) > 1;
+        st.launches = 1 + (second ? 1 : 0) + (pd.rowmax >= 0 ? 1 : 0);
         const void* a = dev(pd.a);
         const void* a2 = pd.a2 >= 0 ? dev(pd.a2) : nullptr;
         const void* b = pd.bDerived ? pd.bDerived : dev(pd.b);

@@ -79,6 +79,7 @@ struct F32MmaParams {
   int tiles_n, tiles_per_batch;
   int num_kb;
   int split;                    // CTAs that share a tile's K range
+  int one_order;                // 64-wide tiles: the small products in one accumulator, in the order of 128-wide ones
   const float* a;
   const float* b;
   long long lda, ldb, a_batch, b_batch;
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
             tc_mma_pair<kMmaF16>(d + BN, a + pa, b, id1, 1u);         // m * h
             tc_mma_pair<kMmaF16>(d + BN, a + pa, b + pb, id1, 1u);    // m * m
             tc_mma_pair<kMmaF16>(d + BN, a + 2 * pa, b, id1, 1u);     // l * h
-          } else if constexpr (BN == 128) {
+          } else if (BN == 128 || (!CONTRACT && p.one_order)) {
             tc_mma<kMmaF16>(d, a, b, id2, go);                        // h * [h | m]
             tc_mma<kMmaF16>(d + BN, a + pa, b, id1, 1u);              // m * h
             tc_mma<kMmaF16>(d + BN, a + pa, b + pb, id1, 1u);         // m * m
@@ -724,7 +725,10 @@ __global__ void __launch_bounds__(kThreads, 1) f32_mma_kernel(const __grid_const
             tmem_ld_wait();
 #pragma unroll
             for (int e = 0; e < 8; e += 2) {
-              const float2 t = add2(__uint_as_float(small[e]), __uint_as_float(small[e + 1]), __uint_as_float(small2[e]), __uint_as_float(small2[e + 1]));
+              // (a third accumulator that was not used holds anything)
+              const bool third = CONTRACT || !p.one_order;
+              const float2 t = add2(__uint_as_float(small[e]), __uint_as_float(small[e + 1]), third ? __uint_as_float(small2[e]) : 0.f,
+                                    third ? __uint_as_float(small2[e + 1]) : 0.f);
               small[e] = __float_as_uint(t.x), small[e + 1] = __float_as_uint(t.y);
             }
           } else {
@@ -918,6 +922,7 @@ struct Choice {
 // (B200, 1.9 GHz): a k-block takes 1700 cycles with 64-wide and 2400 with 128-wide tiles (the loaders) and 3750 on a CTA
 // pair for four times the 128-wide tile's work on two SMs (the rate the tensor pipe sustains); rows that are not 16-byte aligned cost a
 // third more loads.  Everything around the loop: 8800, 11500 and 18000 cycles, and 1500 + 150 per CTA of a K split.
+// (Clusters are counted with the 64-wide kernel: every kernel here leaves room for one CTA per SM.)
 Choice choose_tiles(int m, int n, int num_kb, int batch, bool vec, int bn_override, int split_override, bool pairs, int dev, int sms) {
   Choice best;
   for (int bn = 64; bn <= (pairs ? 256 : 128); bn *= 2) {
@@ -978,9 +983,11 @@ F32MmaTiles f32_mma_tiles(const F32MmaShape& s) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, s.tile_n, s.whole_k ? 1 : 0, !s.short_chains, dev, sms);
+  // A sum's order follows from the tile kind and the split.  64- and 128-wide tiles can share one, pairs and parts cannot.
+  const Choice c = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, s.tile_n, s.whole_k ? 1 : 0,
+                                !s.short_chains && !s.whole_k, dev, sms);
   F32MmaTiles t;
-  t.bn = c.bn, t.split = c.split, t.us = c.cycles / 1900.0;
+  t.bn = c.bn, t.split = c.split, t.us = c.cycles / 1900.0, t.one_order = s.whole_k;
   return t;
 }
 
@@ -994,10 +1001,11 @@ bool f32_mma_faster(const F32MmaShape& s, F32MmaTiles* tiles) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  *tiles = f32_mma_tiles(s);
+  if (tiles->bn == 0) return false;
+  if (s.whole_k) return true;   // (the pre-pass adds in another order)
   const Choice any = choose_tiles(s.m, s.n, (s.k + kBlockK - 1) / kBlockK, s.batch, s.aligned_in, 0, 0, true, dev, sms);
   const double here = any.cycles / 1900.0 * (s.conv ? (any.bn == 256 ? 1.05 : 1.2) : 1.0);   // (gathering pixels costs more)
-  *tiles = f32_mma_tiles(s);
-  if (any.bn == 0 || tiles->bn == 0) return false;
   const double tiles_m = (s.m + 127) / 128;
   auto prepass = [&](int bn, double block_us) {
     const double waves = std::max(1.0, tiles_m * ((s.n + bn - 1) / bn) * s.batch / sms);
@@ -1038,6 +1046,7 @@ int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err)
   cudaGetDevice(&dev);
   const int best_bn = L.tiles.bn;
   p.split = L.tiles.split;
+  p.one_order = L.tiles.one_order;
   p.tiles_n = (L.n + best_bn - 1) / best_bn;
   const int tile_rows = best_bn == 256 ? 256 : 128, share = best_bn == 256 ? 2 * p.split : p.split;
   const long long per_batch = static_cast<long long>((L.m + tile_rows - 1) / tile_rows) * p.tiles_n;

@@ -14,6 +14,7 @@ namespace pmlb {
 struct F32MmaTiles {
   int bn = 64, split = 1;
   double us = 0;
+  bool one_order = false;   // the same additions in the same order whatever the width
 };
 
 // C[b][i][j] = sum_k A(b, i, k) * B(b, k, j), everything fp32 in device memory.
@@ -48,7 +49,7 @@ struct F32MmaShape {
   bool aligned_in = true, aligned_out = true;   // rows start on 16-byte boundaries
   long long elems = 0;                          // elements that each call's pre-pass would split
   int tile_n = 0;                               // 0 = choose; else 64 or 128
-  bool whole_k = false;                         // no K split
+  bool whole_k = false;                         // one order of additions whatever the number of rows and tiles
   bool short_chains = false;                    // no CTA pairs, whose accumulator chains run over all of K
 };
 

@@ -913,7 +913,7 @@ cudaError_t launch_contract(const GenericParams& p, cudaStream_t stream) {
 namespace {
 // Whether a problem goes kRun neighbours per thread, `width` elements of the last dim each.
 bool lean_run_form(const LeanParams& p, int width, LeanRun* r) {
-  if (p.rank < 2 || p.n_src != 2 || p.has_init || p.agg != PMLB_AGG_SUM || p.combo != PMLB_COMBO_MUL) return false;
+  if (p.one_order || p.rank < 2 || p.n_src != 2 || p.has_init || p.agg != PMLB_AGG_SUM || p.combo != PMLB_COMBO_MUL) return false;
   const int along = p.rank - 2;
   const bool move0 = p.src[0].out[along] != 0, move1 = p.src[1].out[along] != 0;
   if (move0 == move1) return false;

@@ -51,6 +51,7 @@ struct GenericParams {
 struct LeanParams {
   int rank, n_src, n_check;
   int agg, combo, has_init, out_dtype, init_dtype;
+  int one_order;                // the same roundings at every size (no runs of neighbours)
   int size[PMLB_MAX_RANK];
   FastDiv fd_size[PMLB_MAX_RANK];
   long long out_stride[PMLB_MAX_RANK];

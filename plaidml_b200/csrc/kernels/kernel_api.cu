@@ -136,6 +136,12 @@ pmlb::ConvGeom conv_geom(const pmlb_conv_desc& d) {
   return g;
 }
 
+// PMLB_SPLIT_K=0 in the environment: sums never depend on the tile count.
+bool sums_in_one_order() {
+  const char* v = std::getenv("PMLB_SPLIT_K");
+  return v && v[0] == '0';
+}
+
 pmlb_status alloc_plan_memory(pmlb_plan* plan, size_t scratch_bytes, bool need_status) {
   cudaGetDevice(&plan->device);
   if (scratch_bytes > 0) {
@@ -245,7 +251,10 @@ size_t pmlb_plan_scratch_bytes(const pmlb_plan* plan) { return plan ? plan->scra
 
 const char* pmlb_plan_kind(const pmlb_plan* plan) { return plan ? plan->kind_name : ""; }
 
-int pmlb_plan_split_k(const pmlb_plan* plan) { return plan ? plan->ksplit : 1; }
+int pmlb_plan_split_k(const pmlb_plan* plan) {
+  if (!plan) return 1;
+  return plan->kind == kPlanGemm && plan->f32_mma ? plan->f32_tiles.split : plan->ksplit;
+}
 
 pmlb_status pmlb_plan_arm_timeout_test(pmlb_plan* plan, int wait_limit_ms) {
   if (!plan || plan->kind != kPlanGemm) return fail(PMLB_ERR_INVALID, "the time-out test takes a gemm plan");
@@ -343,8 +352,7 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
     shape.aligned_out = d->ldc % 4 == 0;
     shape.elems = (a_mats * d->m + b_mats * d->n) * d->k;
     shape.tile_n = d->tile_n;
-    const char* env = std::getenv("PMLB_SPLIT_K");
-    shape.whole_k = (d->flags & PMLB_GEMM_NO_SPLIT_K) != 0 || (env && env[0] == '0');
+    shape.whole_k = (d->flags & PMLB_GEMM_NO_SPLIT_K) != 0 || sums_in_one_order();
     // (a forced 256-wide tile is refused for f32, by the other route)
     if ((d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_faster(shape, &plan->f32_tiles)) {
       plan->f32_mma = true;   // no scratch but the status word
@@ -372,8 +380,7 @@ pmlb_status pmlb_gemm_dispatch(const pmlb_gemm_desc* d, pmlb_plan** out) {
     }
   }
   // Split K?  (8/16-bit inputs read in place, one matrix, no row maxima: see PMLB_GEMM_NO_SPLIT_K)
-  const char* split_env = std::getenv("PMLB_SPLIT_K");   // "0": never split (sums then never depend on the tile count)
-  const bool split_allowed = !(split_env && split_env[0] == '0') || (d->flags & PMLB_GEMM_SPLIT_K);
+  const bool split_allowed = !sums_in_one_order() || (d->flags & PMLB_GEMM_SPLIT_K);
   if (!f32 && !plan->transpose_b && d->batch == 1 && !(d->epilogue & PMLB_EPI_ROWMAX) && d->k_first == 0 &&
       !(d->flags & PMLB_GEMM_NO_SPLIT_K) && split_allowed) {
     const int bk = 128 / eb;
@@ -641,6 +648,7 @@ pmlb_status pmlb_conv_dispatch(const pmlb_conv_desc* d, pmlb_plan** out) {
   shape.aligned_in = shape.aligned_out = d->k % 4 == 0;
   shape.elems = static_cast<long long>(d->n) * d->h * d->w * d->c;
   shape.tile_n = d->tile_n;
+  shape.whole_k = sums_in_one_order();
   pmlb::F32MmaTiles f32_tiles;
   if (f32 && (d->tile_n == 0 || d->tile_n == 64 || d->tile_n == 128) && pmlb::f32_mma_takes_conv(conv_geom(*d)) &&
       pmlb::f32_mma_faster(shape, &f32_tiles)) {
@@ -1085,7 +1093,8 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
     }
   }
   plan->lean = pmlb::lean_form(p, &plan->lean_params);
-  if (pmlb::product_form(p, &plan->product)) {
+  plan->lean_params.one_order = sums_in_one_order();   // (then term by term, whatever the sizes)
+  if (!plan->lean_params.one_order && pmlb::product_form(p, &plan->product)) {
     const pmlb::ProductForm& f = plan->product;
     pmlb::F32MmaShape shape;
     shape.m = static_cast<int>(f.m), shape.n = static_cast<int>(f.n), shape.k = static_cast<int>(f.k), shape.batch = static_cast<int>(f.batch);

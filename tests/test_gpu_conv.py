@@ -2,6 +2,7 @@
 
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from plaidml_b200 import kernels as K
@@ -413,6 +414,34 @@ def test_first_layer_fused_with_its_max_pool(n, h, w, c, r, pad, epi):
     two = oracle.pool2d_nhwc_f32(as_f32(mid), "max", (3, 3), (2, 2), (1, 1), (p // 2, q // 2))
     check_close(got, two, 1e-2)
     assert (got != two).mean() < 0.02
+
+
+@pytest.mark.parametrize("h,c,r,k,stride", [(14, 128, 3, 128, 1), (56, 64, 1, 256, 2), (28, 64, 3, 32, 1)])
+def test_fp32_images_do_not_depend_on_the_others_without_k_split(h, c, r, k, stride, monkeypatch):
+    monkeypatch.setenv("PMLB_SPLIT_K", "0")
+    g = rng(6500 + h)
+    n, pad = 40, r // 2
+    p = out_size(h, r, stride, pad, pad, 1)
+    x, f = dev(g.standard_normal((n, h, h, c)).astype(np.float32)), dev(g.standard_normal((r, r, c, k)).astype(np.float32))
+
+    def images(count):
+        d = K.ConvDesc()
+        d.in_dtype, d.out_dtype = K.F32, K.F32
+        d.n, d.h, d.w, d.c, d.r, d.s, d.k, d.p, d.q = count, h, h, c, r, r, k, p, p
+        d.stride_h = d.stride_w = stride
+        d.pad_h = d.pad_w = pad
+        d.dil_h = d.dil_w = 1
+        plan = K.Plan("conv", d)
+        plan.set_filter(ptr(f), K.F32)
+        out = empty((count, p, p, k), K.F32)
+        xs = x[-count:].contiguous()
+        plan.conv(ptr(xs), ptr(out))
+        plan.check()
+        return out
+
+    whole = images(n)
+    for count in (1, 3, 12):
+        assert torch.equal(images(count), whole[-count:])
 
 
 @pytest.mark.parametrize("n,h,w,c,r,k,stride,pad,epi", [

@@ -534,6 +534,23 @@ def test_f32_split_operands_keep_every_nan(m, n, k, tile_n):
         np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("n,k", [(1000, 2048), (2049, 513), (60, 300), (256, 64)])
+@pytest.mark.parametrize("by_env", [False, True], ids=["flag", "environment"])
+def test_f32_rows_do_not_depend_on_the_others_without_k_split(n, k, by_env, monkeypatch):
+    # K split, 64- and 128-wide tiles, CTA pairs, several waves of few terms: each by the number of rows, unless forbidden
+    if by_env:
+        monkeypatch.setenv("PMLB_SPLIT_K", "0")
+    g = rng(3500 + n)
+    m = 6000
+    a, b = dev(g.standard_normal((1, m, k)).astype(np.float32)), dev(g.standard_normal((1, k, n)).astype(np.float32))
+    flags = 0 if by_env else K.GEMM_NO_SPLIT_K
+    whole = run_gemm(K.F32, K.F32, a, b, m, n, k, 1, False, flags=flags)[0]
+    for rows in (1, 100, 300, 2048):
+        part, _, plan = run_gemm(K.F32, K.F32, a[:, -rows:].contiguous(), b, rows, n, k, 1, False, flags=flags)
+        assert plan.split_k == 1
+        assert torch.equal(part[0], whole[0, -rows:])
+
+
 # --- CTA pairs (two CTAs per 256 x 256 tile) -----------------------------------------------------
 
 @pytest.mark.parametrize("b_is_nk", [True, False], ids=["B[n][k]", "B[k][n]"])

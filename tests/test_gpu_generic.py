@@ -610,6 +610,32 @@ def test_products_of_infinite_and_of_tiny_operands(a, b, c, m, n, k):
     assert np.all(off[fine] <= k * (2.0 ** -24 * np.abs(want[fine]) + 2.0 ** -150))
 
 
+def test_contractions_add_term_by_term_without_k_split(monkeypatch):
+    # a matrix product and a depthwise filter, both large enough for kernels with other roundings
+    monkeypatch.setenv("PMLB_SPLIT_K", "0")
+    g = rng(7500)
+    m, n, k = 90, 70, 33
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 3, 2
+    for i, v in enumerate([m, n, k]):
+        d.range[i] = v
+    d.out = K.make_access(K.F32, [m, n], [{0: 1}, {1: 1}])
+    d.src[0] = K.make_access(K.F32, [k, m], [{2: 1}, {0: 1}])
+    d.src[1] = K.make_access(K.F32, [k, n], [{2: 1}, {1: 1}])
+    out, ref = run_contract(d, [g.standard_normal(s).astype(np.float32) for s in ((k, m), (k, n))], (m, n), K.F32)
+    np.testing.assert_array_equal(out, ref)
+    rows, c, r = 20000, 51, 3      # 5000 runs of 51: wide enough for runs of neighbours
+    d = K.ContractDesc()
+    d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, 3, 2
+    for i, v in enumerate([rows, c, r]):
+        d.range[i] = v
+    d.out = K.make_access(K.F32, [rows, c], [{0: 1}, {1: 1}])
+    d.src[0] = K.make_access(K.F32, [rows + r - 1, c], [{0: 1, 2: 1}, {1: 1}])
+    d.src[1] = K.make_access(K.F32, [r, c], [{2: 1}, {1: 1}])
+    out, ref = run_contract(d, [g.standard_normal(s).astype(np.float32) for s in ((rows + r - 1, c), (r, c))], (rows, c), K.F32)
+    np.testing.assert_array_equal(out, ref)
+
+
 def test_product_that_does_not_cover_its_output_or_reads_out_of_range_stays_exact():
     # a range shorter than the output dim leaves the identity there; one longer than an operand's dim skips terms
     g = rng(7300)
