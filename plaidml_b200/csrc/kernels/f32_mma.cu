@@ -869,6 +869,10 @@ __global__ void __launch_bounds__(256) filter_to_f32_kernel(const In* in, float*
   if (i < n) out[i] = static_cast<float>(in[i]);
 }
 
+// Zero until a launch gives up waiting.  Handed out in turn: two plans 1024 apart share one, and either may then report it.
+constexpr unsigned kStatusWords = 1024;
+__device__ int g_status_words[kStatusWords];
+
 using KernelPtr = void (*)(const F32MmaParams);
 
 // The shared-memory limit is an attribute per device.
@@ -1013,6 +1017,13 @@ bool f32_mma_faster(const F32MmaShape& s, F32MmaTiles* tiles) {
   };
   const double there = std::min(prepass(128, 0.58), prepass(64, 0.38));
   return here <= 0.95 * there;
+}
+
+int* f32_mma_status_word() {
+  static std::atomic<unsigned> next{0};
+  void* words = nullptr;
+  if (cudaGetSymbolAddress(&words, g_status_words) != cudaSuccess) return nullptr;
+  return static_cast<int*>(words) + next.fetch_add(1, std::memory_order_relaxed) % kStatusWords;
 }
 
 int f32_mma_launch(const F32MmaLaunch& L, cudaStream_t stream, std::string* err) {

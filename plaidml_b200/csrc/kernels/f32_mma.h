@@ -59,6 +59,10 @@ F32MmaTiles f32_mma_tiles(const F32MmaShape& shape);
 // Whether the kernel is expected to be faster than splitting the operands into TF32 parts by pre-passes, and its tiles.
 bool f32_mma_faster(const F32MmaShape& shape, F32MmaTiles* tiles);
 
+// A status word of the library's own on the current device, for plans that hold no device memory (so that they can be made
+// and freed while a stream is being captured, and a captured graph outlive its plan); null if the device has none to give.
+int* f32_mma_status_word();
+
 // Returns 0 on success, otherwise a pmlb_status value with a message in *err.
 int f32_mma_launch(const F32MmaLaunch& launch, cudaStream_t stream, std::string* err);
 

@@ -1103,11 +1103,15 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
     plan->f32_tiles = pmlb::f32_mma_tiles(shape);
     plan->f32_mma = plan->f32_tiles.bn != 0 && pmlb::product_pays(f, plan->lean, plan->f32_tiles.us);
   }
-  pmlb_status st = alloc_plan_memory(plan, 0, plan->f32_mma);
-  if (st != PMLB_OK) {
-    pmlb_plan_free(plan);
-    return st;
+  if (plan->f32_mma) {
+    plan->status = pmlb::f32_mma_status_word();
+    plan->owns_status = false;
+    if (!plan->status) {
+      delete plan;
+      return cuda_fail(cudaGetLastError(), "contract: status word");
+    }
   }
+  cudaGetDevice(&plan->device);
   *out = plan;
   return PMLB_OK;
 }

@@ -636,6 +636,42 @@ def test_contractions_add_term_by_term_without_k_split(monkeypatch):
     np.testing.assert_array_equal(out, ref)
 
 
+def test_contraction_plans_are_made_and_freed_while_a_stream_is_captured():
+    # a matrix product and a strided contraction; the graph outlives the plans
+    m, n, k = 160, 96, 700
+    x, y = torch.randn(k, m, device="cuda"), torch.randn(k, n, device="cuda")
+    s = torch.randn(n, device="cuda")
+    out, scaled = torch.zeros(m, n, device="cuda"), torch.zeros(m, n, device="cuda")
+
+    def desc(src_b, b, n_idx):
+        d = K.ContractDesc()
+        d.agg, d.combo, d.n_idx, d.n_src = K.AGG_SUM, K.COMBO_MUL, n_idx, 2
+        for i, v in enumerate([m, n, k][:n_idx]):
+            d.range[i] = v
+        d.out = K.make_access(K.F32, [m, n], [{0: 1}, {1: 1}])
+        d.src[0] = K.make_access(K.F32, [k, m], [{2: 1}, {0: 1}]) if n_idx == 3 else d.out
+        d.src[1] = K.make_access(K.F32, src_b, b)
+        return d
+
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        product = K.Plan("contract", desc([k, n], [{2: 1}, {1: 1}], 3))
+        product.contract([ptr(x), ptr(y)], ptr(out), stream=stream.cuda_stream)
+        scale = K.Plan("contract", desc([n], [{1: 1}], 2))
+        scale.contract([ptr(out), ptr(s)], ptr(scaled), stream=stream.cuda_stream)
+        del product, scale
+    for _ in range(2):
+        x.normal_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want = x.double().t() @ y.double()
+        assert torch.linalg.norm(out.double() - want) <= 1e-6 * torch.linalg.norm(want)
+        assert torch.equal(scaled, out * s)
+
+
 def test_product_that_does_not_cover_its_output_or_reads_out_of_range_stays_exact():
     # a range shorter than the output dim leaves the identity there; one longer than an operand's dim skips terms
     g = rng(7300)
