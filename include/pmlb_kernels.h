@@ -96,7 +96,9 @@ pmlb_status pmlb_plan_check(pmlb_plan* plan, void* stream);
  * plans.  pmlb_plan_check then reads that word. */
 pmlb_status pmlb_plan_share_status(pmlb_plan* plan, int* device_word);
 
-/* Name of the kernel family a plan resolved to ("tc_gemm", "tc_conv", "row_reduce", ...). */
+/* Name of the kernel family a plan resolved to ("tc_gemm", "tc_conv", "row_reduce", ...).  Contractions:
+ * "generic_contract_product" (an f32 matrix product, on the tensor cores), "generic_contract_strided" (offsets by steps) or
+ * "generic_contract". */
 const char* pmlb_plan_kind(const pmlb_plan* plan);
 /* Parts the K range of a GEMM plan is split into (1 = a single pass): by two passes for 8/16-bit inputs, among the CTAs of
  * a cluster within one launch for fp32. */

@@ -1396,6 +1396,9 @@ class Planner {
     st.kernel = "generic_contract";
     st.detail = (op.label.empty() ? std::string("contract") : op.label) + " -> " + outShape.str() +
                 (why.empty() ? "" : " [" + why + "]");
+    const std::string kind = pmlb_plan_kind(plan);
+    if (kind == "generic_contract_product") st.detail += " (f32 product on the tensor cores)";
+    if (kind == "generic_contract_strided") st.detail += " (strided form)";
     void* out = dev(op.result);
     const void* s0 = srcPtrs[0];
     const void* s1 = srcPtrs[1];

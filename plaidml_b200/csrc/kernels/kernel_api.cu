@@ -1014,7 +1014,6 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
   pmlb_plan* plan = new (std::nothrow) pmlb_plan();
   if (!plan) return fail(PMLB_ERR_INVALID, "out of host memory");
   plan->kind = kPlanContract;
-  plan->kind_name = "generic_contract";
   pmlb::GenericParams& p = plan->generic;
   std::memset(&p, 0, sizeof(p));
   p.agg = d->agg;
@@ -1103,6 +1102,7 @@ pmlb_status pmlb_contract_dispatch(const pmlb_contract_desc* d, pmlb_plan** out)
     plan->f32_tiles = pmlb::f32_mma_tiles(shape);
     plan->f32_mma = plan->f32_tiles.bn != 0 && pmlb::product_pays(f, plan->lean, plan->f32_tiles.us);
   }
+  plan->kind_name = plan->f32_mma ? "generic_contract_product" : (plan->lean ? "generic_contract_strided" : "generic_contract");
   if (plan->f32_mma) {
     plan->status = pmlb::f32_mma_status_word();
     plan->owns_status = false;

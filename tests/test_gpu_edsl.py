@@ -103,6 +103,24 @@ def test_contraction_whose_indices_only_sums_and_differences_bound():
     np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-6)
 
 
+def test_plan_text_names_the_route_of_a_contraction():
+    g = rng(1262)
+    x, y, s = (g.standard_normal(sh).astype(np.float32) for sh in ((300, 64), (300, 48), (64, 48)))
+    X, Y, S = (Placeholder(DType.FLOAT32, list(v.shape)) for v in (x, y, s))
+    i, j, k = TensorIndexes(3)
+    grad = Contraction().outShape(64, 48).outAccess(i, j).sum(X[k, i] * Y[k, j]).build()
+    scaled = Contraction().outShape(64, 48).outAccess(i, j).sum(grad[i, j] * S[i, j]).build()
+    spread = Contraction().outShape(64, 48).outAccess(i, j).sum(scaled[i // 2, j]).build()
+    runner = Runner(Program("routes", [X, Y, S], [grad, scaled, spread]), "cuda.0")
+    lines = [ln for ln in runner.executable.describe().splitlines() if "generic_contract" in ln]
+    assert len(lines) == 3
+    assert "tensor cores" in lines[0] and "strided form" in lines[1] and "(" not in lines[2], lines
+    got = runner.run([x, y, s])
+    want = x.astype(np.float64).T @ y.astype(np.float64)
+    np.testing.assert_allclose(got[0], want, atol=1e-5 * np.abs(want).max())
+    np.testing.assert_array_equal(got[1], got[0] * s)
+
+
 def test_run_on_adopted_caller_memory():
     # buffers that borrow the caller's (pageable) numpy memory, as the reference's C++ Buffer(ptr, shape) does:
     # inputs are read from it and outputs land in it
