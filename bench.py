@@ -393,7 +393,7 @@ def extras(device: str, local_rank: int, peaks: dict) -> dict:
     write_gbs = (1 << 30) / best / 1e6
     out["hbm_write_only"] = {"gbs": write_gbs, "what": "fill of a 1 GiB device buffer, best of 5 (CUDA events)"}
 
-    # cfg1: fp32 1024^3 via 3xTF32
+    # cfg1: fp32 1024^3
     g = np.random.Generator(np.random.PCG64(1234 + 1))
     A, B, C = progs.tile_gemm(DType.FLOAT32, 1024, 1024, 1024)
     r = Runner(Program("cfg1", [A, B], [C]), device)
@@ -405,11 +405,11 @@ def extras(device: str, local_rank: int, peaks: dict) -> dict:
     err = float(np.max(np.abs(got[rows] - want)) / np.max(np.abs(want)))
     sp = timed(r)
     tf = 2 * 1024**3 / sp["mean_ms"] / 1e9
-    # three TF32 products per fp32 product, TF32 at half the bf16 rate
+    # six bf16 part products per fp32 product
     out["cfg1_fp32_gemm_1024"] = {
         **sp, "tflops": tf, "kernels": r.executable.launch_count, "check": {"rows_vs_f64": err, "ok": err < 1e-5},
         "roofline": {"bound": "tensor", "achieved": tf, "peak": burst / 6.0, "unit": "TFLOP/s", "frac": tf / (burst / 6.0),
-                     "traffic": None, "peak_source": "bf16_tflops / 6: TF32 runs at half the bf16 rate and an fp32 product is three TF32 products"}}
+                     "traffic": None, "peak_source": "bf16_tflops / 6: an fp32 product is six bf16 part products"}}
 
     # bf16 4096^3 Tile GEMM
     g = np.random.Generator(np.random.PCG64(1234 + 6))

@@ -407,7 +407,7 @@ cudaError_t launch_pack_rows(const void* in, void* out, int n, int h, int w, int
   const long long rows = static_cast<long long>(n) * h;
   const long long total = rows * wp * (cp / 8);
   if (total <= 0) return cudaSuccess;
-  pack_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(      static_cast<const uint16_t*>(in), static_cast<uint4*>(out), rows, w, c, wp, cp / 8, pad_w);
+  pack_rows_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(static_cast<const uint16_t*>(in), static_cast<uint4*>(out), rows, w, c, wp, cp / 8, pad_w);
   return cudaGetLastError();
 }
 

@@ -9,7 +9,7 @@ launches of the kernel of interest:
 
     i8_4k      int8 -> int32 Tile GEMM 4096^3            (tc_contract_kernel, int8, B as [k][n])
     bf16_4k    bf16 Tile GEMM 4096^3, f32 accumulate     (tc_contract_kernel, bf16)
-    f32_1k     fp32 Tile GEMM 1024^3 via three TF32 products
+    f32_1k     fp32 Tile GEMM 1024^3
     bf16_2a    bf16 GEMM 50176 x 256 x 1024 (the shape of ResNet-50's res4x_2a layers at 256 images: A streamed once)
     bf16_2c    bf16 GEMM 50176 x 1024 x 256 (res4x_2c: short K, 103 MB of output)
     conv3      conv 3x3 56x56 64->64 + bias + ReLU, batch 16

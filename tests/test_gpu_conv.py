@@ -454,10 +454,13 @@ def test_fp32_images_do_not_depend_on_the_others_without_k_split(h, c, r, k, str
     (2, 8, 8, 32, 3, 32, 2, 1, K.EPI_BIAS | K.EPI_RESIDUAL | K.EPI_RELU),     # 32 output pixels in all: one ragged tile
     (2, 8, 8, 32, 3, 32, 2, 1, K.EPI_BIAS | K.EPI_RESIDUAL),
     (2, 8, 8, 32, 3, 32, 2, 1, K.EPI_BIAS),
+    (33, 14, 15, 256, 1, 512, 1, 0, K.EPI_BIAS | K.EPI_RELU),   # CTA pairs, the last one's second tile partly there
+    (16, 14, 14, 256, 3, 256, 1, 1, K.EPI_BIAS | K.EPI_RESIDUAL | K.EPI_RELU),   # CTA pairs, K in four parts
+    (12, 13, 15, 256, 3, 256, 1, 1, 0),                         # 128-wide tiles, K in three parts
 ])
 def test_fp32_convolution_on_tensor_cores(n, h, w, c, r, k, stride, pad, epi):
-    # fp32 activations and filter: three TF32 products per term on the im2col route (activation and filter split into
-    # high and low parts by pre-passes), f32 accumulation; against the oracle's f64-accumulated loop nest to 1e-5
+    # fp32 activations and filter, split into bf16 parts inside the kernel (3 channels: into TF32 parts by pre-passes), f32
+    # accumulation; against the oracle's f64-accumulated loop nest to 1e-5
     g = rng(6100 + h + c)
     p, q = out_size(h, r, stride, pad, pad, 1), out_size(w, r, stride, pad, pad, 1)
     x = g.uniform(-1, 1, size=(n, h, w, c)).astype(np.float32)

@@ -67,7 +67,7 @@ def test_reference_microkernel_known_answers():
 
 def test_small_fp32_gemm_is_exact_like_the_reference_expects():
     # plaidml/edsl/examples/gemm.cc GEMM_FLOAT32 is checked with checkExact in the reference: any true f32
-    # arithmetic reproduces it bit for bit (three TF32 products per term would not)
+    # arithmetic reproduces it bit for bit (part products on the tensor cores would not)
     kat = next(k for k in KATS if k["name"] == "GEMM_FLOAT32")
     program = P.GOLDEN_BUILDERS["GEMM_FLOAT32"]()
     ins = [np.array(v, dtype=np.float32).reshape(3, 3) for v in kat["inputs"]]
@@ -440,8 +440,8 @@ def test_strided_shortcut_projection_runs_inside_the_blocks_last_layer():
 
 
 def test_fp32_network_layers_run_on_tensor_cores():
-    # the reference's own networks are fp32 (networks/oplib/resnet50.cc): its convolutions take the im2col route as three
-    # TF32 products per term, 1x1 stride-1 layers the fp32 GEMM; nothing falls to the general kernel; 1e-5 like the fp32 GEMM
+    # the reference's own networks are fp32 (networks/oplib/resnet50.cc): its convolutions run on the tensor cores as part
+    # products, 1x1 stride-1 layers as the fp32 GEMM; nothing falls to the general kernel; 1e-5 like the fp32 GEMM
     g = rng(1264)
     n = 2
     x = g.uniform(-1, 1, (n, 32, 32, 3)).astype(np.float32)

@@ -133,7 +133,7 @@ def test_reference_sources_run_on_the_cuda_device():
         res = subprocess.run([str(OUT / "ref_run")], capture_output=True, text=True, timeout=600, env=env)
         assert res.returncode == 0 and "Running..." in res.stdout and "tile.contract" in res.stdout, (res.stdout[-1500:], res.stderr[-1500:])
     if (OUT / "ref_layer").exists():
-        # N K C H W R S stride: a 3 x 3 convolution on 56 x 56 x 64 in fp32 (the tensor-core route with three TF32 products)
+        # N K C H W R S stride: a 3 x 3 convolution on 56 x 56 x 64 in fp32 (on the tensor cores)
         res = subprocess.run([str(OUT / "ref_layer"), "8", "64", "64", "56", "56", "3", "3", "1"], capture_output=True, text=True,
                              timeout=600, env=env)
         assert res.returncode == 0 and "Running..." in res.stdout and "conv2d:8:64:64:56:56:3:3:1" in res.stdout, \
