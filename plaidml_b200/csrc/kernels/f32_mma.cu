@@ -6,9 +6,9 @@
 // positive terms).  Error of a single product against 64 bits, in norm: 3.0e-8 (5.1e-8 with m cut; plain f32 2.5e-8,
 // three TF32 products 6.6e-8), of sums of 8 to 4096 terms 0.6 to 0.2 times that of plain f32 sums.  bf16 parts end at
 // 2^-133: operands below 2^-110 lose what lies under 2^-134 (2^-16 of themselves at 2^-118).
-// bf16 MMAs run at twice the TF32 rate, so six of them cost what three TF32 products
-// cost, but the parts keep all 24 bits (two TF32 parts keep 22), occupy 6 bytes of shared memory per element instead
-// of 8, and bf16 operands may be MN-major, so a [k][n] B or a transposed A needs no transposition.
+// bf16 MMAs run at twice the TF32 rate, so six of them cost what three TF32 products cost, but three parts keep 24 bits
+// (two TF32 parts 22), occupy 6 bytes of shared memory per element instead of 8, and bf16 operands may be MN-major, so a
+// [k][n] B or a transposed A needs no transposition.
 //
 // One CTA computes a 128 x BN tile (or the part of its K range that falls to it, see below):
 //   warps 0..15  loaders: fp32 from global memory into registers one operand tile ahead, cut into the three parts,
@@ -37,8 +37,8 @@
 // 4096 x 4096 51.8 -> 49.3, 301 x 303 x 305 7.0 -> 7.4): problems of 6 to 12 us gave up to 0.4 us for it.
 // CTA pairs: the rate the tensor pipe sustains under the power limit (six products of 2048 x 2048 x 1024 in 41 us:
 // 1.27 PFLOP/s, 1.6 in the loop).  Small problems: ~6 us of launch, first loads, last sums and stores.
-// Measured (graph replays), split copies by a pre-pass -> here: 1 x 1000 x 2048 35 -> 11.5 us, 300^3 12.9 -> 7.1, 1024^3
-// 22.0 -> 18.2, 256 x 4096 x 4096 96 -> 49, 512 x 512 x 4096 62 -> 22, 1999 x 2001 x 1001 71 -> 49; convolutions 8 x 28 x
+// Measured (graph replays), split copies by a pre-pass -> here: 1 x 1000 x 2048 35 -> 11.4 us, 300^3 12.9 -> 6.9, 1024^3
+// 22.0 -> 18.1, 256 x 4096 x 4096 96 -> 49, 512 x 512 x 4096 62 -> 22, 1999 x 2001 x 1001 71 -> 49; convolutions 8 x 28 x
 // 28 x 128 -> 128, 3x3 25.5 -> 20.0, 32 x 7 x 7 x 512 -> 512, 3x3 63 -> 45 (pairs, K in parts), 1 x 7 x 7 x 512 61 -> 15.
 // Walking several tiles per CTA with the stores behind the next tile's loads was slower (1024^3 21.2 us against 19.2).
 //
