@@ -586,6 +586,32 @@ def test_f32_rows_do_not_depend_on_the_others_without_k_split(n, k, by_env, monk
         assert torch.equal(part[0], whole[0, -rows:])
 
 
+@pytest.mark.parametrize("in_dtype,out_dtype", [(K.BF16, K.BF16), (K.BF16, K.F32), (K.F16, K.F16), (K.I8, K.I32), (K.I8, K.I8), (K.F32, K.F32)])
+@pytest.mark.parametrize("n,ldc", [(67, 80), (130, 144), (257, 272), (96, 112), (63, 64)])
+def test_columns_behind_a_result_stay_as_they_are(in_dtype, out_dtype, n, ldc):
+    # the result is a block of columns of a wider matrix whose rows start on 16-byte boundaries
+    m, k, batch = 140, 64, 2
+    make = lambda *sh: torch.randint(-3, 4, sh, device="cuda").to(empty((1,), in_dtype).dtype)
+    a, b = make(batch, m, k), make(batch, n, k)
+    wide = torch.full((batch, m, ldc), 77, dtype=empty((1,), out_dtype).dtype, device="cuda")
+    d = K.GemmDesc()
+    d.in_dtype, d.out_dtype = in_dtype, out_dtype
+    d.m, d.n, d.k, d.batch = m, n, k, batch
+    d.lda, d.ldb, d.ldc = k, k, ldc
+    d.stride_a, d.stride_b, d.stride_c = m * k, n * k, m * ldc
+    d.b_is_nk = 1
+    plan = K.Plan("gemm", d)
+    plan.gemm(ptr(a), ptr(b), ptr(wide))
+    plan.check()
+    want = a.double() @ b.double().transpose(1, 2)     # (small whole numbers)
+    if out_dtype == K.I8:
+        want = (want.long() + 128) % 256 - 128
+    elif out_dtype in (K.BF16, K.F16):
+        want = want.to(wide.dtype)
+    assert torch.equal(wide[:, :, :n].double(), want.double())
+    assert torch.all(wide[:, :, n:] == 77)
+
+
 # --- CTA pairs (two CTAs per 256 x 256 tile) -----------------------------------------------------
 
 @pytest.mark.parametrize("b_is_nk", [True, False], ids=["B[n][k]", "B[k][n]"])
