@@ -681,7 +681,7 @@ int tc_launch(const TcLaunch& L, cudaStream_t stream, std::string* err) {
     bool fast = (ob == 2 || ob == 4) && (ob == ob_tmpl || no_store);
     if (L.out != nullptr) {
       // A TMA store writes whole 16-byte units of a row: zeros over what the caller has behind a ragged last one.  (Only
-      // that chunk stored element by element from the staging buffer: ResNet-50 643 -> 653 us, and no faster itself.)
+      // that chunk stored element by element from the staging buffer: ResNet-50 648 -> 658 us, and no faster itself.)
       fast = fast && aligned16(L.out) && (L.ldc * ob) % 16 == 0 && (static_cast<long long>(L.n) * ob) % 16 == 0 &&
              (L.batch == 1 || (L.out_batch_stride * ob) % 16 == 0);
     }
